@@ -80,6 +80,9 @@ constexpr int kBlock = 256;
 // default L2 prefetch distance of the fused kernel: 54% of one resident wave
 // (148 SMs x 5 blocks -> ~400 blocks), the best of a sweep at 512x256x256
 constexpr int kPrefetchWavePct = 54;
+// the same for the direct-planes step, which fetches only the flag words: 27%
+// (200 blocks), the middle of a flat range of 100-300
+constexpr int kHeadsWavePct = 27;
 inline int grid_for(long long n, int block = kBlock) { return (int)((n + block - 1) / block); }
 
 enum BcKind { BC_NS_VEL_EQ, BC_NS_VEL_NEQ, BC_NS_PRESSURE, BC_NS_BOUNCEBACK, BC_AD_DIRICHLET, BC_AD_PULSE, BC_AD_NEUMANN };
@@ -143,8 +146,10 @@ struct fm_lattice {
     uint32_t* cellw = nullptr;          // per-cell flag words (k_build_flags)
     bool dirty = true;                  // flags / fusion need rebuilding
     bool split_open = false;            // a step begun by fm_step_planes, not yet finished
+    bool chain = false;                 // within fm_step: the last queued work is a step kernel the next one may chain to
     int fuse_outlet = 0, fuse_neumann = 0, fuse_dirichlet = 0;
     uint32_t pf_dist = 0;               // L2 prefetch distance of the fused kernel (blocks)
+    uint32_t pf_full = 0;               // the same for the in-lane planes' kernels
     bool pf_set = false;                // pf_dist fixed by fm_set_tuning
     double rho_out = 1.0, c_in = 0.0;
     bool profiling = false;
@@ -444,47 +449,53 @@ int prepare(fm_lattice* L)
 {
     if (!L->dirty) return FM_OK;
     const int nx = L->p.nx;
-    // a full x = nx-1 plane can be fused when its x-1 neighbour is always the
-    // previous lane of the same warp: every row ends at an odd cell index,
-    // which holds for even nx
-    const bool lanes_ok = nx >= 3 && nx % 2 == 0;
-    L->fuse_outlet = 0;
-    if (lanes_ok && L->ns_post.size() == 1 && L->ns_post[0].kind == BC_NS_PRESSURE &&
-        is_full_x_plane(L, L->ns_post[0], nx - 1)) {
-        L->fuse_outlet = 1;
-        L->rho_out = L->ns_post[0].v[0];
-    }
-    L->fuse_neumann = 0;
-    L->fuse_dirichlet = 0;
-    {
-        int nd = 0, nn = 0;
-        bool planes = true;
-        for (const Bc& b : L->ad_post) {
-            if (b.kind == BC_AD_DIRICHLET) { ++nd; planes = planes && is_full_x_plane(L, b, 0); }
-            else { ++nn; planes = planes && is_full_x_plane(L, b, nx - 1); }
+    // Which boundary planes the step kernel can take.  The in-lane planes
+    // (coupled_cell) need the x-1 neighbour of x = nx-1 in the previous lane of
+    // the same warp, and x = 0 and 1 side by side: every row starting at an
+    // even cell index, which holds for even nx.  The direct planes
+    // (coupled_cell_direct) need neither, but their own conditions
+    // (direct_planes): odd nx fuses all its planes with them or none.  Against
+    // the list path's five extra launches, 125x83x71 (FP32) went from 73.5 to
+    // 33 us a step.
+    const bool even = nx % 2 == 0;
+    auto fuse = [&](bool lanes_ok) {
+        L->fuse_outlet = 0;
+        if (lanes_ok && L->ns_post.size() == 1 && L->ns_post[0].kind == BC_NS_PRESSURE &&
+            is_full_x_plane(L, L->ns_post[0], nx - 1)) {
+            L->fuse_outlet = 1;
+            L->rho_out = L->ns_post[0].v[0];
         }
-        // the in-kernel AD planes need every AD update in the fused kernel:
-        // no cell may be deferred behind a list-path NS boundary
-        const bool no_deferred = L->fuse_outlet || L->ns_post.empty();
-        if (planes && nd <= 1 && nn <= 1 && lanes_ok && no_deferred) {
+        L->fuse_neumann = 0;
+        L->fuse_dirichlet = 0;
+        {
+            int nd = 0, nn = 0;
+            bool planes = true;
             for (const Bc& b : L->ad_post) {
-                if (b.kind == BC_AD_DIRICHLET) { L->fuse_dirichlet = 1; L->c_in = b.v[0]; }
-                else L->fuse_neumann = 1;
+                if (b.kind == BC_AD_DIRICHLET) { ++nd; planes = planes && is_full_x_plane(L, b, 0); }
+                else { ++nn; planes = planes && is_full_x_plane(L, b, nx - 1); }
+            }
+            // the in-kernel AD planes need every AD update in the fused kernel:
+            // no cell may be deferred behind a list-path NS boundary
+            const bool no_deferred = L->fuse_outlet || L->ns_post.empty();
+            if (planes && nd <= 1 && nn <= 1 && lanes_ok && no_deferred) {
+                for (const Bc& b : L->ad_post) {
+                    if (b.kind == BC_AD_DIRICHLET) { L->fuse_dirichlet = 1; L->c_in = b.v[0]; }
+                    else L->fuse_neumann = 1;
+                }
             }
         }
-    }
-    // the NEQ inlet plane: the x = 1 lane computes next step's x = 0 values in
-    // the fused kernel; needs its final populations, so no list-path NS
-    // boundary may rewrite x = 1 after the collision
-    L->fuse_inlet = 0;
-    if (lanes_ok && L->ns_pre.size() == 1 && L->ns_pre[0].kind == BC_NS_VEL_NEQ &&
-        is_full_x_plane(L, L->ns_pre[0], 0) && (L->fuse_outlet || L->ns_post.empty())) {
-        L->fuse_inlet = 1;
-        if (!L->x0post) {
-            L->rows_stride = (uint32_t)(((long long)L->p.ny * L->p.nz + 31) / 32 * 32);
-            int rc0 = dev_alloc((char**)&L->x0post, (size_t)19 * L->rows_stride * L->elt, L->stream);
-            if (rc0) return rc0;
-        }
+        // the NEQ inlet plane: the x = 1 cells compute next step's x = 0 values in
+        // the fused kernel; needs their final populations, so no list-path NS
+        // boundary may rewrite x = 1 after the collision
+        L->fuse_inlet = lanes_ok && L->ns_pre.size() == 1 && L->ns_pre[0].kind == BC_NS_VEL_NEQ &&
+                        is_full_x_plane(L, L->ns_pre[0], 0) && (L->fuse_outlet || L->ns_post.empty());
+    };
+    fuse(even ? nx >= 3 : nx >= fm::kDirectMinNx);
+    if (!even && L->fuse_outlet != L->fuse_neumann) fuse(false);
+    if (L->fuse_inlet && !L->x0post) {
+        L->rows_stride = (uint32_t)(((long long)L->p.ny * L->p.nz + 31) / 32 * 32);
+        int rc0 = dev_alloc((char**)&L->x0post, (size_t)19 * L->rows_stride * L->elt, L->stream);
+        if (rc0) return rc0;
     }
     // deferred AD cells: those a non-fused post-stream NS boundary rewrites
     dev_free(L->deferred, L->stream);
@@ -527,15 +538,16 @@ int prepare(fm_lattice* L)
         L->collision == FM_COLL_BGK);
     FM_CHECK_LAUNCH("k_build_flags");
     if (!L->pf_set) {
-        // FP32: about half a resident wave ahead.  FP64 and the 16-bit forms:
-        // none.  Measured on 33.5M-cell lattices of three shapes, the prefetch
-        // made FP64 17-20% and the 16-bit forms 5-9% slower; on 4M-cell
-        // lattices it gained at most 4% (FP64, 40 blocks) and 1% (16-bit).
+        // Direct planes: the flag words a quarter of a resident wave ahead, for
+        // every form (fm::prefetch_heads).  The in-lane planes' kernels fetch
+        // everything a block reads (fm::prefetch_ahead): FP32 half a wave ahead;
+        // FP64 and the 16-bit forms not at all, which that made 5-20% slower.
         int dev = 0, sms = 148;
         const int per_sm = 5;   // resident 256-thread blocks at 48 registers
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        L->pf_dist = L->elt == 4 ? (uint32_t)(kPrefetchWavePct * sms * per_sm / 100) : 0u;
+        L->pf_dist = (uint32_t)(kHeadsWavePct * sms * per_sm / 100);
+        L->pf_full = L->elt == 4 ? (uint32_t)(kPrefetchWavePct * sms * per_sm / 100) : 0u;
     }
     L->dirty = false;
     return FM_OK;
@@ -597,6 +609,7 @@ fm::StepArgs<T, QT> make_args(const fm_lattice* L)
     a.neg_zero = (typename fm::Pop<T>::R)-0.0;
     a.status = L->d_status;
     a.st_rows = 0;
+    a.outputs = 1;
     return a;
 }
 
@@ -718,20 +731,56 @@ bool wide_offsets(const fm_lattice* L)
     return 18LL * L->ns + (long long)L->p.nx * L->p.ny + 2LL * L->p.nx + 1 >= (1LL << 31);
 }
 
-template <typename T, typename QT, bool POROUS, bool MON>
-void launch_coupled(const fm_lattice* L, int grid, cudaStream_t st, const fm::StepArgs<T, QT>& a)
+// The fused planes written by their inward neighbours (fm::coupled_cell_direct):
+// when the pressure outlet and the AD Neumann outlet are both fused or both
+// absent, for rows that fit a warp's staging slots.
+template <typename T, typename QT>
+bool direct_planes(const fm::StepArgs<T, QT>& a)
 {
-    if constexpr (fm::Pop<T>::kShifted) {
-        if (wide_offsets(L)) {
-            fm::k_coupled_step<T, QT, POROUS, MON, true><<<grid, kBlock, 0, st>>>(a);
+    return a.fuse_outlet == a.fuse_neumann && a.nx >= fm::kDirectMinNx;
+}
+
+// `chained`: the previous work on `st` is a direct-planes step kernel of the
+// same run of steps, so this one may start while that one drains (programmatic
+// dependent launch; the kernel waits for it before its first pull).  Measured
+// 2-4 us a step, what a launch and the first and last blocks' ramps cost: FP32
+// 32x16x16 6.2 -> 4.2 us, 128x64x64 24.6 -> 22.3, 256x128x128 164 -> 161.
+template <typename T, typename QT, bool POROUS, bool MON>
+void launch_coupled(const fm_lattice* L, int grid, cudaStream_t st, const fm::StepArgs<T, QT>& a, bool chained = false)
+{
+    if constexpr (!MON) {
+        if (direct_planes(a)) {
+            void (*kern)(const fm::StepArgs<T, QT>) = fm::k_coupled_step<T, QT, POROUS, false, false, true>;
+            if constexpr (fm::Pop<T>::kShifted) {
+                if (wide_offsets(L)) kern = fm::k_coupled_step<T, QT, POROUS, false, true, true>;
+            }
+            cudaLaunchAttribute attr{};
+            attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr.val.programmaticStreamSerializationAllowed = 1;
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3((unsigned)grid);
+            cfg.blockDim = dim3(kBlock);
+            cfg.stream = st;
+            cfg.attrs = &attr;
+            cfg.numAttrs = chained ? 1 : 0;
+            cudaLaunchKernelEx(&cfg, kern, a);   // errors: the caller's FM_CHECK_LAUNCH
             return;
         }
     }
-    fm::k_coupled_step<T, QT, POROUS, MON><<<grid, kBlock, 0, st>>>(a);
+    fm::StepArgs<T, QT> al = a;
+    al.pf_dist = L->pf_full;
+    if constexpr (fm::Pop<T>::kShifted) {
+        if (wide_offsets(L)) {
+            fm::k_coupled_step<T, QT, POROUS, MON, true><<<grid, kBlock, 0, st>>>(al);
+            return;
+        }
+    }
+    fm::k_coupled_step<T, QT, POROUS, MON><<<grid, kBlock, 0, st>>>(al);
 }
 
+// `last`: nothing of this fm_step call follows the step but its sample
 template <typename T, typename QT>
-int launch_step(fm_lattice* L)
+int launch_step(fm_lattice* L, bool last)
 {
     using R = typename fm::Pop<T>::R;
     const long long s = L->step + 1;
@@ -765,7 +814,8 @@ int launch_step(fm_lattice* L)
         fm::k_ad_fill<T><<<grid_for(b.count), kBlock, 0, st>>>(gA, L->ns, b.cells, b.count, phi_in, (R)L->g_shift);
     }
     // the fused NS + coupling + LDF + AD step
-    const fm::StepArgs<T, QT> a = make_args<T, QT>(L);
+    fm::StepArgs<T, QT> a = make_args<T, QT>(L);
+    a.outputs = last;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     if (L->profiling) {
         if (L->prof_used + 2 > L->prof_ev.size()) {
@@ -795,10 +845,13 @@ int launch_step(fm_lattice* L)
         fm::StepArgs<T, QT> am = a;
         am.mon = L->d_mon_part;
         grid = grid_for(L->n);
+        const bool chained = L->chain && !L->profiling;
         if (mon && bgk) launch_coupled<T, QT, false, true>(L, grid, st, am);
         else if (mon) launch_coupled<T, QT, true, true>(L, grid, st, am);
-        else if (bgk) launch_coupled<T, QT, false, false>(L, grid, st, a);
-        else launch_coupled<T, QT, true, false>(L, grid, st, a);
+        else if (bgk) launch_coupled<T, QT, false, false>(L, grid, st, a, chained);
+        else launch_coupled<T, QT, true, false>(L, grid, st, a, chained);
+        // the next step may chain to this one when nothing else is queued between them
+        L->chain = !mon && direct_planes(a) && fm_launches_per_step(L) == 1;
     }
     if (ev1) FM_CUDA(cudaEventRecord(ev1, st));
     if (mon) {
@@ -931,6 +984,7 @@ int probe_into(fm_lattice* L, double* dst)
 
 int take_sample(fm_lattice* L)
 {
+    L->chain = false;
     if (!L->nprobe) return FM_OK;
     int rc = ensure_bt_capacity(L, L->bt_count + 1);
     if (rc) return rc;
@@ -1118,7 +1172,9 @@ int convert_layout(fm_lattice* L, int to)
     return fail(FM_ERR_STATE, "pair layout: 16-bit forms only");
 }
 
-template <typename T, typename QT> struct StepOp { static int run(fm_lattice* L) { return launch_step<T, QT>(L); } };
+template <typename T, typename QT> struct StepOp {
+    static int run(fm_lattice* L, bool last) { return launch_step<T, QT>(L, last); }
+};
 template <typename T, typename QT> struct PlanesOp {
     static int run(fm_lattice* L, int z0, int z1) { return launch_planes<T, QT>(L, z0, z1); }
 };
@@ -1161,6 +1217,15 @@ int ensure_layout(fm_lattice* L)
         want = 1;
     if (want == L->layout) return FM_OK;
     return dispatch<LayoutOp>(L, want);
+}
+
+// One launch per step with every boundary plane a form the batches, the step
+// monitor, the adjoint and the split steps know: for odd nx (whose planes only
+// the direct planes fuse) none of them.
+bool one_launch_in_lanes(fm_lattice* L)
+{
+    if (fm_launches_per_step(L) != 1) return false;
+    return L->p.nx % 2 == 0 || !(L->fuse_inlet || L->fuse_outlet || L->fuse_dirichlet || L->fuse_neumann);
 }
 
 int add_bc(fm_lattice* L, std::vector<Bc>& into, Bc b, const std::vector<int>& cells, const std::vector<int>* nei)
@@ -1581,13 +1646,14 @@ int fm_step(fm_lattice* L, int nsteps)
     int prc = prepare(L);
     if (!prc) prc = ensure_layout(L);
     if (prc) return prc;
-    if (L->mon_every > 0 && fm_launches_per_step(L) != 1)
+    if (L->mon_every > 0 && !one_launch_in_lanes(L))
         return fail(FM_ERR_UNSUPPORTED, "fm_step: the step monitor needs every boundary inside the fused step");
     if (L->fuse_inlet && L->inlet_state == 0) prc = dispatch<InletFusedOp>(L);
     else if (!L->fuse_inlet && L->inlet_state == 1) prc = dispatch<InletPlainOp>(L);
     if (prc) return prc;
+    L->chain = false;
     for (int i = 0; i < nsteps; ++i) {
-        int rc = dispatch<StepOp>(L);
+        int rc = dispatch<StepOp>(L, i + 1 == nsteps);
         if (rc) return rc;
         if (L->nprobe && L->probe_every > 0 && L->step % L->probe_every == 0) {
             rc = take_sample(L);
@@ -2063,7 +2129,7 @@ int fm_set_prefetch_distance(fm_lattice* L, int blocks)
     if (check_lattice(L)) return FM_ERR_ARG;
     if (blocks < 0) { L->pf_set = false; L->dirty = true; return FM_OK; }
     L->pf_set = true;
-    L->pf_dist = (uint32_t)blocks;
+    L->pf_dist = L->pf_full = (uint32_t)blocks;
     return FM_OK;
 }
 
@@ -2155,19 +2221,23 @@ int batch_upload_const(fm_batch* B)
     return FM_OK;
 }
 
+// `last`: the batch's outputs may be read before its next step
 template <typename T, typename QT>
-int batch_launch_step(fm_batch* B, int parity)
+int batch_launch_step(fm_batch* B, int parity, bool last)
 {
     if (B->mode == 3) {
         const auto* args = reinterpret_cast<const fm::StepArgs<T, QT>*>(B->h_args[parity].data());
         FM_CUDA(cudaEventRecord(B->fork_ev, B->stream));
         for (int k = 0; k < fm_batch::kSideStreams; ++k) FM_CUDA(cudaStreamWaitEvent(B->side[k], B->fork_ev, 0));
+        bool chain[fm_batch::kSideStreams] = {};   // the stream's last work is a direct-planes step of this loop
         for (size_t i = 0; i < B->lats.size(); ++i) {
-            cudaStream_t st = B->side[B->side_of[i]];
-            if (B->collision == FM_COLL_BGK)
-                fm::k_coupled_step<T, QT, false><<<grid_for(B->lats[i]->n), kBlock, 0, st>>>(args[i]);
-            else
-                fm::k_coupled_step<T, QT, true><<<grid_for(B->lats[i]->n), kBlock, 0, st>>>(args[i]);
+            const int k = B->side_of[i];
+            fm::StepArgs<T, QT> a = args[i];
+            a.outputs = last;
+            const int grid = grid_for(B->lats[i]->n);
+            if (B->collision == FM_COLL_BGK) launch_coupled<T, QT, false, false>(B->lats[i], grid, B->side[k], a, chain[k]);
+            else launch_coupled<T, QT, true, false>(B->lats[i], grid, B->side[k], a, chain[k]);
+            chain[k] = direct_planes(a);
         }
         FM_CHECK_LAUNCH("k_coupled_step (batch)");
         for (int k = 0; k < fm_batch::kSideStreams; ++k) {
@@ -2199,7 +2269,7 @@ template <typename T, typename QT> struct BatchConstOp {
     static int run(fm_lattice*, fm_batch* B) { return batch_upload_const<T, QT>(B); }
 };
 template <typename T, typename QT> struct BatchStepOp {
-    static int run(fm_lattice*, fm_batch* B, int parity) { return batch_launch_step<T, QT>(B, parity); }
+    static int run(fm_lattice*, fm_batch* B, int parity, bool last) { return batch_launch_step<T, QT>(B, parity, last); }
 };
 
 template <typename T, typename QT>
@@ -2227,7 +2297,7 @@ template <typename T, typename QT> struct BatchGridOp {
 
 int batch_dispatch_items(fm_batch* B) { return dispatch<BatchItemsOp>(B->lats[0], B); }
 int batch_dispatch_grid(fm_batch* B) { return dispatch<BatchGridOp>(B->lats[0], B); }
-int batch_dispatch_step(fm_batch* B, int parity) { return dispatch<BatchStepOp>(B->lats[0], B, parity); }
+int batch_dispatch_step(fm_batch* B, int parity, bool last) { return dispatch<BatchStepOp>(B->lats[0], B, parity, last); }
 int batch_dispatch_const(fm_batch* B)
 {
     return (B->mode == 1 || B->mode == 2) ? dispatch<BatchConstOp>(B->lats[0], B) : FM_OK;
@@ -2312,9 +2382,9 @@ int batch_launch_probes(fm_batch* B)
 }
 
 // one step of every lattice; `s` is the step number being completed
-int batch_one(fm_batch* B, long long s, int parity)
+int batch_one(fm_batch* B, long long s, int parity, bool last)
 {
-    int rc = batch_dispatch_step(B, parity);
+    int rc = batch_dispatch_step(B, parity, last);
     if (rc) return rc;
     if (B->probe_every > 0 && s % B->probe_every == 0) return batch_launch_probes(B);
     return FM_OK;
@@ -2359,7 +2429,7 @@ int fm_batch_create(fm_lattice* const* lattices, int count, void* stream, fm_bat
         if (L->step != L0->step) return fail(FM_ERR_STATE, "fm_batch_create: lattices are at different steps");
         if (L->elt == 2 && wide_offsets(L))
             return fail(FM_ERR_UNSUPPORTED, "fm_batch_create: a 16-bit lattice of more than ~119M cells steps on its own");
-        if (fm_launches_per_step(L) != 1)
+        if (!one_launch_in_lanes(L))
             return fail(FM_ERR_UNSUPPORTED, "fm_batch_create: a lattice needs boundary kernels besides the fused "
                                             "step (full x-plane boundaries and even Nx are required)");
         const int every = (L->nprobe && L->probe_every > 0) ? L->probe_every : 0;
@@ -2483,7 +2553,7 @@ int fm_batch_step(fm_batch* B, int nsteps)
     // batch's before its launches (and again inside its graph)
     if ((rc = batch_dispatch_const(B))) return rc;
     auto single = [&]() -> int {
-        int r = batch_one(B, s + 1, parity);
+        int r = batch_one(B, s + 1, parity, left == 1);
         ++s;
         parity ^= 1;
         --left;
@@ -2498,7 +2568,7 @@ int fm_batch_step(fm_batch* B, int nsteps)
             FM_CUDA(cudaStreamBeginCapture(B->stream, cudaStreamCaptureModeThreadLocal));
             int rc2 = batch_dispatch_const(B);
             for (long long i = 0; i < G && !rc2; ++i)
-                rc2 = batch_one(B, i + 1, (int)((parity + i) & 1));
+                rc2 = batch_one(B, i + 1, (int)((parity + i) & 1), i + 1 == G);
             cudaError_t e = cudaStreamEndCapture(B->stream, &g);
             if (rc2) { if (g) cudaGraphDestroy(g); return rc2; }
             if (e != cudaSuccess) return fail(FM_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
@@ -2596,10 +2666,10 @@ int fm_batch_autotune(fm_batch* B, int trial_steps, int* mode, int* block, int* 
                 if (!rc) rc = batch_dispatch_const(B);
                 if (rc) break;
                 int parity = B->lats[0]->cur;
-                for (int i = 0; i < 2 && !rc; ++i, parity ^= 1) rc = batch_dispatch_step(B, parity);
+                for (int i = 0; i < 2 && !rc; ++i, parity ^= 1) rc = batch_dispatch_step(B, parity, true);
                 if (rc) break;
                 cudaEventRecord(e0, B->stream);
-                for (int i = 0; i < trials && !rc; ++i, parity ^= 1) rc = batch_dispatch_step(B, parity);
+                for (int i = 0; i < trials && !rc; ++i, parity ^= 1) rc = batch_dispatch_step(B, parity, true);
                 cudaEventRecord(e1, B->stream);
                 if (cudaEventSynchronize(e1) != cudaSuccess) { rc = fail(FM_ERR_CUDA, "autotune sync failed"); break; }
                 float ms = 0.0f;
@@ -2707,10 +2777,10 @@ int adj_forward(AdjCtx& X, const AdjState& in, AdjState& out)
     a.fB = (T*)out.f; a.gB = (T*)out.g;
     a.phi = (R*)out.phi; a.q = (QT*)out.q;
     a.x0post = (T*)X.x0scratch;
-    a.pf_dist = 0;
+    a.outputs = 0;   // the recomputed states are read in the fused representation only
     ++X.forward_steps;
-    if (L->collision == FM_COLL_BGK) fm::k_coupled_step<T, QT, false><<<grid_for(L->n), kBlock, 0, L->stream>>>(a);
-    else fm::k_coupled_step<T, QT, true><<<grid_for(L->n), kBlock, 0, L->stream>>>(a);
+    if (L->collision == FM_COLL_BGK) launch_coupled<T, QT, false, false>(L, grid_for(L->n), L->stream, a);
+    else launch_coupled<T, QT, true, false>(L, grid_for(L->n), L->stream, a);
     FM_CHECK_LAUNCH("adjoint forward");
     return FM_OK;
 }
@@ -2973,7 +3043,7 @@ int fm_adjoint_breakthrough(fm_lattice* L, int nsteps, const double* target, int
         for (size_t i = 0; i < h.size(); ++i)
             if (h[i] != nx - 1 + nx * (int)i) return fail(FM_ERR_UNSUPPORTED, "fm_adjoint_breakthrough: the outlet probe must be the x = nx-1 plane");
     }
-    if (fm_launches_per_step(L) != 1 || !L->ad_pre.empty())
+    if (!one_launch_in_lanes(L) || !L->ad_pre.empty())
         return fail(FM_ERR_UNSUPPORTED, "fm_adjoint_breakthrough: only fused full-plane boundaries (even nx, no pulse) are differentiated");
     if (!L->ns_pre.empty() && !L->fuse_inlet)
         return fail(FM_ERR_UNSUPPORTED, "fm_adjoint_breakthrough: NS inlet must be the fused NEQ plane");
@@ -3127,7 +3197,7 @@ int fm_step_planes(fm_lattice* L, int z0, int z1)
         int rc = prepare(L);
         if (!rc) rc = ensure_layout(L);
         if (rc) return rc;
-        if (fm_launches_per_step(L) != 1)
+        if (!one_launch_in_lanes(L))
             return fail(FM_ERR_UNSUPPORTED, "fm_step_planes: the step needs boundary kernels besides the fused one");
         // launches over planes keep the warps of a whole-lattice launch:
         // plane starts at a multiple of 32 cells (and 32 words of the pair layout)

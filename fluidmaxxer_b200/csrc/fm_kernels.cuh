@@ -259,6 +259,9 @@ constexpr uint32_t kDeferred = 1u << 20;  // AD update runs after the post-strea
 constexpr uint32_t kFaceYZ = 1u << 21;    // y = 0, y = ny-1, z = 0 or z = nz-1
 constexpr uint32_t kXLo = 1u << 22;       // x = 0
 constexpr uint32_t kXHi = 1u << 23;       // x = nx-1
+constexpr uint32_t kXLo1 = 1u << 24;      // x = 1
+constexpr uint32_t kXHi1 = 1u << 25;      // x = nx-2
+constexpr uint32_t kXEdge = kXLo | kXHi | kXLo1 | kXHi1;
 
 // division by an invariant divisor d: q = floor(c * M / 2^64) with
 // M = ceil(2^64 / d) is exact for every 32-bit c (M = 0 encodes d = 1)
@@ -328,6 +331,7 @@ struct StepArgs {
     R neg_zero;                           // -0, a value the code generator cannot see (fm_pair.cuh)
     uint32_t st_rows;                     // staged pair kernel: x-rows per tile (fm_pair.cuh)
     int* __restrict__ status;             // device status word: bit 0 a shared-memory stage wait gave up
+    int outputs;                          // x0post of this step may be read before the next step (direct planes)
 };
 
 // The step monitor: FP64 sums over the cells of a launch of the post-step
@@ -390,6 +394,15 @@ __device__ __forceinline__ void l2_prefetch(const void* p, uint32_t bytes)
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
+// Programmatic dependent launch: a grid launched with that attribute may start
+// while its predecessor drains; pdl_wait returns once the predecessor has
+// ended and its writes are visible (at once in a grid launched without it).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch_dependents()
+{
+    asm volatile("griddepcontrol.launch_dependents;");
+}
+
 // The first warp of a block prefetches into L2 everything the block
 // `pf_dist` blocks ahead reads at its own cells: the 19 + 7 population planes
 // of buffer A, the flag words, phi, q and the optional per-cell fields.  Pulls
@@ -413,6 +426,28 @@ __device__ __forceinline__ void prefetch_ahead(const StepArgs<T, QT>& a)
     else if (lane == 28 && a.isotherm) l2_prefetch(a.q + c0, cnt * (uint32_t)sizeof(QT));
     else if (lane == 29 && a.porosity) l2_prefetch(a.porosity + c0, cnt * (uint32_t)sizeof(R));
     else if (lane == 30 && a.tau_ad) l2_prefetch(a.tau_ad + c0, cnt * (uint32_t)sizeof(R));
+}
+
+// Prefetches of the direct-planes step: the loads that head or end the chain
+// flag word -> pulls -> collision -> C(s-1), q -> transport.  One thread of a
+// block fetches the flag words pf_dist blocks ahead (the pulls' addresses wait
+// for them), and a cell in the adsorption region asks for its C(s-1) and q
+// before its pulls, so the three trips to DRAM overlap.  Fetching the
+// populations ahead as prefetch_ahead does costs more than it saves here:
+// FP32 512x256x128 613 us a step with it, 595 with no distance, 586 with the
+// flag words 100-300 blocks ahead (588 at 800 and 592 without the C and q
+// prefetch); FP16 160x96x96 50.4 -> 47.8, FP64 106.2 -> 103.1.
+template <typename T, typename QT>
+__device__ __forceinline__ void prefetch_heads(const StepArgs<T, QT>& a, uint32_t c, uint32_t w)
+{
+    if (threadIdx.x == 0 && a.pf_dist) {
+        const uint32_t c0 = a.c_first + (blockIdx.x + a.pf_dist) * blockDim.x;
+        if (c0 < a.ns) l2_prefetch(a.cellw + c0, min((uint32_t)blockDim.x, a.ns - c0) * 4u);
+    }
+    if (a.isotherm && (w & kRegion)) {
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(a.phi + c));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(a.q + c));
+    }
 }
 
 // neighbour coordinates of a cell with the reference's mapCoord rule
@@ -743,11 +778,17 @@ __device__ __forceinline__ typename Pop<T>::R ad_collide(const StepArgs<T, QT>& 
 }
 
 template <typename T, typename QT>
-__device__ __forceinline__ void store7(const StepArgs<T, QT>& a, uint32_t c, const typename Pop<T>::R* gn)
+__device__ __forceinline__ void store7(const StepArgs<T, QT>& a, uint32_t c, const typename Pop<T>::R* gn,
+                                       uint32_t draw)
 {
     T* const p = a.gB + c;
 #pragma unroll
-    for (int k = 0; k < 7; ++k) PopG<T>::st(p + (size_t)k * a.ns, gn[k], k, a.g_shift, c);
+    for (int k = 0; k < 7; ++k) PopG<T>::st(p + (size_t)k * a.ns, gn[k], k, a.g_shift, draw);
+}
+template <typename T, typename QT>
+__device__ __forceinline__ void store7(const StepArgs<T, QT>& a, uint32_t c, const typename Pop<T>::R* gn)
+{
+    store7(a, c, gn, c);   // the rounding's draw is the cell's own
 }
 
 // direction sets as bit masks, for per-lane (runtime) direction indices
@@ -950,6 +991,46 @@ __device__ __forceinline__ void dev_ns_collide(const StepArgs<T, QT>& a, uint32_
     dev_ns_collide_por<T, QT, POROUS>(a, w, POROUS ? __ldg(a.porosity + c) : 0.0f, h, vx, vy, vz);
 }
 
+// the LDF source and the D3Q7 collision of the 16-bit forms (src/collision/ADBGKCollision.cu:95-124)
+template <typename T, typename QT>
+__device__ __forceinline__ float dev_ad_collide(const StepArgs<T, QT>& a, uint32_t c, uint32_t w, const float* gi,
+                                                float vx, float vy, float vz, bool commit, float* gn)
+{
+    const float S = ldf_source(a, c, w, commit);
+    float ph = gi[0];
+#pragma unroll
+    for (int k = 1; k < 7; ++k) ph += gi[k];
+    ph = fmaxf(ph, a.min_conc);
+    const float om = a.tau_ad ? __frcp_rn(__ldg(a.tau_ad + c)) : a.omega_ad;
+    const float wp0 = 0.25f * ph, wp1 = 0.125f * ph, ws0 = 0.25f * S, ws1 = 0.125f * S;
+#pragma unroll
+    for (int k = 0; k < 7; ++k) {
+        float eu;
+        if (k == 0) eu = 0.0f;
+        else if (k == 1) eu = vx;
+        else if (k == 2) eu = -vx;
+        else if (k == 3) eu = vy;
+        else if (k == 4) eu = -vy;
+        else if (k == 5) eu = vz;
+        else eu = -vz;
+        const float wp = k == 0 ? wp0 : wp1;
+        const float geq = fmaf(4.0f * wp, eu, wp);
+        gn[k] = fmaf(om, geq - gi[k], gi[k] + (k == 0 ? ws0 : ws1));
+    }
+    return ph;
+}
+
+// the D3Q7 update in the storage's own form
+template <typename T, typename QT>
+__device__ __forceinline__ typename Pop<T>::R ad_update(const StepArgs<T, QT>& a, uint32_t c, uint32_t w,
+                                                        const typename Pop<T>::R* gi, typename Pop<T>::R ux,
+                                                        typename Pop<T>::R uy, typename Pop<T>::R uz, bool commit,
+                                                        typename Pop<T>::R* gn)
+{
+    if constexpr (Pop<T>::kShifted) return dev_ad_collide(a, c, w, gi, ux, uy, uz, commit, gn);
+    else return ad_collide(a, c, w, gi, ux, uy, uz, commit, gn);
+}
+
 template <typename T, typename QT, bool POROUS, bool MON = false, bool WIDE = false>
 __device__ __forceinline__ void coupled_cell_dev(const StepArgs<T, QT>& a, uint32_t cg, MonAcc* mon = nullptr)
 {
@@ -1015,28 +1096,8 @@ __device__ __forceinline__ void coupled_cell_dev(const StepArgs<T, QT>& a, uint3
 
     // ---- LDF source and D3Q7 collision (src/collision/ADBGKCollision.cu:95-124) ----
     const bool do_ad = active && !(w & kDeferred);
-    const float S = ldf_source(a, c, w, do_ad);
-    float ph = gi[0];
-#pragma unroll
-    for (int k = 1; k < 7; ++k) ph += gi[k];
-    ph = fmaxf(ph, a.min_conc);
-    const float om = a.tau_ad ? __frcp_rn(__ldg(a.tau_ad + c)) : a.omega_ad;
-    const float wp0 = 0.25f * ph, wp1 = 0.125f * ph, ws0 = 0.25f * S, ws1 = 0.125f * S;
     float gn[7];
-#pragma unroll
-    for (int k = 0; k < 7; ++k) {
-        float eu;
-        if (k == 0) eu = 0.0f;
-        else if (k == 1) eu = vx;
-        else if (k == 2) eu = -vx;
-        else if (k == 3) eu = vy;
-        else if (k == 4) eu = -vy;
-        else if (k == 5) eu = vz;
-        else eu = -vz;
-        const float wp = k == 0 ? wp0 : wp1;
-        const float geq = fmaf(4.0f * wp, eu, wp);
-        gn[k] = fmaf(om, geq - gi[k], gi[k] + (k == 0 ? ws0 : ws1));
-    }
+    const float ph = dev_ad_collide(a, c, w, gi, vx, vy, vz, do_ad, gn);
     if (a.fuse_neumann && xedge) {
         float left[7];
 #pragma unroll
@@ -1182,6 +1243,244 @@ __device__ __forceinline__ void coupled_cell(const StepArgs<T, QT>& a, uint32_t 
     if (a.fuse_inlet && xedge) fused_inlet(a, c, c, x, active);
 }
 
+// ---------------------------------------------------------------------------
+// The cell update with direct boundary planes.  What a boundary cell takes
+// from its inward neighbour is written by the neighbour's warp, from the
+// neighbour's registers:
+//   x = nx-2  writes the outlet cell's 19 equilibria (one direction per lane);
+//             its seven D3Q7 populations go to the outlet lane by shuffle
+//             (ADNeumannOutlet), or, where that is in the next warp, to memory;
+//   x = 1     writes the x = 0 cell's VelocityDirichletNEQ values of the next
+//             step (one direction per lane; its 19 populations pass through
+//             shared memory, DirectStage);
+//   x = 0     saves its post-collision populations to the x0post side plane,
+//             on steps whose outputs may be read (StepArgs::outputs).
+// No lane reads another cell's stores, so a boundary cell and its neighbour may
+// lie in different warps or blocks (odd nx), and the chain store -> reload ->
+// inlet of coupled_cell is gone.  A boundary cell whose neighbour is a lane of
+// the same warp also stores its own populations, overwritten after a
+// __syncwarp: the first stores then fill whole sectors (without them 128x64x64
+// took 25.8 against 24.6 us a step).  Where the neighbour is in another warp
+// nothing orders the two stores, so the boundary cell leaves its populations out.
+// Stores of single elements into sectors of their own are what the planes
+// cost: of FP16 512x256x128's 519 us, 9 went with the x0post saves of every
+// step and 6 with the outlet's D3Q7 stores; the 38 left per row are worth
+// another 20.  Forming the planes before the row is stored, in registers, would
+// save those, but the registers it takes made every warp slower (FP32 608
+// against 581 us, also with a copy of the code of its own).
+// Applies to rows of 16 cells up, and when the pressure outlet and the AD
+// Neumann outlet are both fused or both absent: an outlet cell advected on its
+// own would need the neighbour's velocity before its own D3Q7 collision.
+// ---------------------------------------------------------------------------
+
+// h_k of the outlet plane for a runtime direction k (dev_outlet)
+__device__ __forceinline__ float dev_outlet_dyn(int k, float rho_out, float drho_out, float ux, float uy, float uz)
+{
+    const float cx = (float)((int)((kPX >> k) & 1u) - (int)((kMX >> k) & 1u));
+    const float cy = (float)((int)((kPY >> k) & 1u) - (int)((kMY >> k) & 1u));
+    const float cz = (float)((int)((kPZ >> k) & 1u) - (int)((kMZ >> k) & 1u));
+    const float m15u2 = -1.5f * fmaf(ux, ux, fmaf(uy, uy, uz * uz));
+    const float e = cx * ux + cy * uy + cz * uz;
+    return fmaf(rho_out * w19<float>(k), fmaf(e, fmaf(4.5f, e, 3.0f), m15u2), drho_out * w19<float>(k));
+}
+
+// value of direction k as the next step reads it back (16-bit: rounded)
+template <typename T>
+__device__ __forceinline__ typename Pop<T>::R stored_value(typename Pop<T>::R v, int k, typename Pop<T>::R fsh)
+{
+    if constexpr (Pop<T>::kShifted) return stored16<T>(v) + fshift<T>(k, fsh);
+    else return v;
+}
+
+// Staging of one warp's boundary rows in shared memory: the x = 1 cell's stored
+// populations and the x = nx-2 cell's velocity of up to kDirectSlots rows (a
+// warp holds 31 / nx + 1 cells of one x at most, so rows of 16 cells up).
+// Written while the populations are in registers, used at the end of the
+// kernel when little else is live: with the planes formed in between, FP64
+// spilled 120 B and FP32 24 B per thread.
+constexpr int kDirectSlots = 2;
+constexpr int kDirectMinNx = 16;
+static_assert(31 / kDirectMinNx + 1 <= kDirectSlots, "a warp's boundary rows fit its staging slots");
+template <typename R>
+struct DirectStage {
+    R in[kDirectSlots][20];    // populations of the x = 1 cells
+    R out[kDirectSlots][20];   // x = nx-2 cells: velocity, or populations (outlet_from_stored)
+};
+
+// The 16-bit forms' outlet for odd nx is formed from the stored (rounded)
+// populations of x = nx-2 in the reference's evaluation order, and its D3Q7
+// codes are those of x = nx-2 bit for bit: what the boundary kernels over cell
+// lists give.  For even nx it follows from the velocity in registers.
+template <typename T>
+__device__ __forceinline__ bool outlet_from_stored(int nx)
+{
+    return Pop<T>::kShifted && (nx & 1);
+}
+
+template <typename T, typename QT>
+__device__ __forceinline__ void direct_stage(const StepArgs<T, QT>& a, uint32_t near0, uint32_t nearn,
+                                             const typename Pop<T>::R* fn, typename Pop<T>::R ux,
+                                             typename Pop<T>::R uy, typename Pop<T>::R uz,
+                                             DirectStage<typename Pop<T>::R>& st)
+{
+    using R = typename Pop<T>::R;
+    const int lane = threadIdx.x & 31;
+    const uint32_t below = (1u << lane) - 1u;
+    const bool in = (near0 >> lane) & 1u, out = (nearn >> lane) & 1u;
+    if (in) {
+        R* const d = st.in[__popc(near0 & below)];
+#pragma unroll
+        for (int k = 0; k < 19; ++k) d[k] = stored_value<T>(fn[k], k, a.f_shift);
+    }
+    if (out) {
+        R* const d = st.out[__popc(nearn & below)];
+        if (outlet_from_stored<T>(a.nx)) {
+#pragma unroll
+            for (int k = 0; k < 19; ++k) d[k] = stored_value<T>(fn[k], k, a.f_shift);
+        } else {
+            d[0] = ux; d[1] = uy; d[2] = uz;
+        }
+    }
+}
+
+// Outlet and inlet populations of the staged rows; cw is the cell of lane 0.
+// The __syncwarp orders them after the boundary cells' own stores.
+template <typename T, typename QT>
+__device__ __forceinline__ void direct_planes(const StepArgs<T, QT>& a, uint32_t near0, uint32_t nearn, uint32_t cw,
+                                              const DirectStage<typename Pop<T>::R>& st)
+{
+    using R = typename Pop<T>::R;
+    const uint32_t lane = threadIdx.x & 31;
+    __syncwarp();
+    if (lane >= 19) return;
+    const uint32_t plane = lane * a.ns + cw;   // direction `lane` of lane 0's cell
+    int slot = 0;
+    for (uint32_t m = nearn; m; m &= m - 1u, ++slot) {
+        T* const p = a.fB + (plane + (uint32_t)__ffs(m));   // x = nx-1: the lane after
+        R ox = st.out[slot][0], oy = st.out[slot][1], oz = st.out[slot][2];
+        if constexpr (Pop<T>::kShifted) {
+            if (outlet_from_stored<T>(a.nx)) {
+                macro_velocity(st.out[slot], ox, oy, oz);
+                Pop<T>::st(p, feq_outlet_dyn(lane, a.rho_out, ox, oy, oz), fshift<T>(lane, a.f_shift));
+            } else {
+                Pop<T>::st_raw(p, dev_outlet_dyn(lane, a.rho_out, a.rho_out - a.rho0, ox, oy, oz));
+            }
+        } else {
+            Pop<T>::st_raw(p, feq_outlet_dyn(lane, a.rho_out, ox, oy, oz));
+        }
+    }
+    slot = 0;
+    for (uint32_t m = near0; m; m &= m - 1u, ++slot) {
+        // the sums of src/core/Macros.cu:40-60, every lane for itself (the reads are broadcasts)
+        R r, jx, jy, jz;
+        moments19(st.in[slot], r, jx, jy, jz, Seq19{});
+        const R inv = (r > R(0)) ? (R(1) / r) : R(0);
+        const R feqN = feq19_dyn(lane, r, jx * inv, jy * inv, jz * inv);
+        const R feqB = feq19_dyn(lane, r, a.uin_x, a.uin_y, a.uin_z);
+        Pop<T>::st(a.fB + (plane + (uint32_t)__ffs(m) - 2u), feqB + (st.in[slot][lane] - feqN),   // x = 0: the lane before
+                   fshift<T>(lane, a.f_shift));
+    }
+}
+
+template <typename T, typename QT, bool POROUS, bool WIDE = false>
+__device__ __forceinline__ void coupled_cell_direct(const StepArgs<T, QT>& a, uint32_t cg,
+                                                    DirectStage<typename Pop<T>::R>& st)
+{
+    using R = typename Pop<T>::R;
+    constexpr bool DEV = Pop<T>::kShifted;   // deviation-form update (coupled_cell_dev)
+    const bool active = cg < a.c_end;
+    const uint32_t c = active ? cg : a.c_end - 1u;
+    const uint32_t w = __ldg(a.cellw + c);   // constant over a run of steps: read ahead of the previous step's end
+    pdl_wait();
+    prefetch_heads(a, c, w);
+    R gi[7], fn[19];
+    const bool xedge = __any_sync(0xffffffffu, w & kXEdge);
+    if (__any_sync(0xffffffffu, w & kFaceYZ)) {
+        int x, y, z;
+        cell_xyz(c, a.nx, a.ny, a.div_nx, a.div_nxy, x, y, z);
+        const Nbr nb(x, y, z, a.nx, a.ny, a.nz, a.px, a.py, a.pz);
+        pull7(a, c, nb, gi);
+        pull19_all<T, !POROUS, DEV>(fn, a.fA, a.ns, c, nb, w, DEV ? R(0) : a.f_shift, Seq19{});
+    } else {
+        using Off = std::conditional_t<!DEV || WIDE, uint32_t, int>;   // pull19_fast
+        const Off ns = (Off)a.ns;
+        const int nxy = a.nx * a.ny;
+        const uint32_t lk = (!POROUS && (w & kSolid)) ? 0x7fffeu : w;
+        if (xedge) {
+            const bool xlo = (w & kXLo) != 0u, xhi = (w & kXHi) != 0u;
+            pull7_fast_all<T>(gi, a.gA + c, ns, a.nx, nxy, a.px, xlo, xhi, a.g_shift, Seq7{});
+            pull19_fast_all<T, !POROUS, DEV>(fn, a.fA + c, ns, a.nx, nxy, a.px, xlo, xhi, lk, R(0), Seq19{});
+        } else {   // x-face selects compiled out
+            pull7_fast_all<T, false>(gi, a.gA + c, ns, a.nx, nxy, a.px, false, false, a.g_shift, Seq7{});
+            pull19_fast_all<T, !POROUS, DEV, false>(fn, a.fA + c, ns, a.nx, nxy, a.px, false, false, lk, R(0),
+                                                    Seq19{});
+        }
+    }
+    R ux = R(0), uy = R(0), uz = R(0);   // velocity of the post-collision populations
+    if constexpr (DEV) {
+        dev_ns_collide<T, QT, POROUS>(a, c, w, fn, ux, uy, uz);
+    } else {
+        ns_collide<T, QT, POROUS>(a, c, w, fn);
+        if (a.coupling || a.fuse_outlet) macro_velocity(fn, ux, uy, uz);
+    }
+    // the next step's grid may take its places: its blocks wait for this grid's end
+    // before their pulls.  Triggered here, not at the start: blocks placed beside
+    // running ones pile up on few SMs (64x32x32: 8.2 against 4.9 us a step)
+    pdl_launch_dependents();
+    bool st_own = active;                // the lane stores its own cell's f and g
+    uint32_t near0 = 0u, nearn = 0u;     // lanes at x = 1 (inlet) and x = nx-2 (outlet)
+    if (xedge) {
+        const int lane = threadIdx.x & 31;
+        const bool inlet = a.fuse_inlet && (w & kXLo);
+        if (inlet && active && a.outputs) {
+            // the stored populations; the 16-bit forms' pass through their shift, as
+            // coupled_cell saves them, where that kernel takes over (even nx)
+            T* const p = a.x0post + fastdiv(c, a.div_nx);
+            const R sh = DEV && (a.nx & 1) == 0 ? a.f_shift : R(0);
+#pragma unroll
+            for (int k = 0; k < 19; ++k)
+                Pop<T>::st(p + (size_t)k * a.rows_stride, stored_value<T>(fn[k], k, sh), fshift<T>(k, sh));
+        }
+        near0 = __ballot_sync(0xffffffffu, active && a.fuse_inlet && (w & kXLo1));
+        nearn = __ballot_sync(0xffffffffu, active && a.fuse_outlet && (w & kXHi1));
+        direct_stage(a, near0, nearn, fn, ux, uy, uz, st);
+        st_own = active && !(inlet && lane == 31) && !(a.fuse_outlet && (w & kXHi) && lane == 0);
+    }
+    if (st_own) {
+        T* const p = a.fB + c;
+#pragma unroll
+        for (int k = 0; k < 19; ++k) Pop<T>::st_raw(p + (size_t)k * a.ns, fn[k]);
+    }
+    if (!a.coupling) ux = uy = uz = R(0);
+
+    const bool do_ad = !(w & kDeferred);
+    R gn[7];
+    const R ph = ad_update(a, c, w, gi, ux, uy, uz, active && do_ad, gn);
+    uint32_t draw = c;   // the cell of the D3Q7 rounding's draw
+    if (xedge) {
+        if (a.fuse_dirichlet && (w & kXLo)) {
+#pragma unroll
+            for (int k = 0; k < 7; ++k) gn[k] = a.c_in * w7<R>(k);
+        }
+        if (a.fuse_neumann) {
+            const bool outlet = (w & kXHi) != 0u;
+            if (active && (w & kXHi1) && (threadIdx.x & 31) == 31) store7(a, c + 1u, gn, c);   // odd nx only
+#pragma unroll
+            for (int k = 0; k < 7; ++k) {
+                const R left = __shfl_up_sync(0xffffffffu, gn[k], 1);
+                if (outlet) gn[k] = left;
+            }
+            if (outlet && outlet_from_stored<T>(a.nx)) draw = c - 1u;
+        }
+    }
+    if (do_ad && active) {
+        // an outlet cell whose neighbour is in another warp leaves g to it
+        if (!(a.fuse_neumann && (w & kXHi) && (threadIdx.x & 31) == 0)) store7(a, c, gn, draw);
+        a.phi[c] = ph;
+    }
+    if (xedge && (near0 | nearn)) direct_planes(a, near0, nearn, cg - (threadIdx.x & 31), st);
+}
+
 // resident 256-thread blocks per SM the step kernel is compiled for: 5 (at
 // most 51 registers) for 4- and 2-byte populations; FP64 needs its 80
 template <typename T>
@@ -1189,11 +1488,17 @@ constexpr int kStepBlocks = sizeof(T) == 8 ? 3 : 5;
 
 // WIDE: unsigned pull offsets in the 16-bit cell update, for lattices too
 // large for signed ones (FP32 and FP64 always use unsigned offsets)
-template <typename T, typename QT, bool POROUS, bool MON = false, bool WIDE = false>
+// DIRECT: boundary planes written by the inward neighbours (coupled_cell_direct)
+template <typename T, typename QT, bool POROUS, bool MON = false, bool WIDE = false, bool DIRECT = false>
 __global__ void __launch_bounds__(256, kStepBlocks<T>) k_coupled_step(const StepArgs<T, QT> a)
 {
-    prefetch_ahead(a);
-    if constexpr (MON) {
+    if constexpr (!DIRECT) prefetch_ahead(a);
+    if constexpr (DIRECT) {
+        static_assert(!MON, "the step monitor sums the outlet cells in their own lanes");
+        __shared__ DirectStage<typename Pop<T>::R> stage[8];   // one per warp of the block
+        coupled_cell_direct<T, QT, POROUS, WIDE>(a, a.c_first + blockIdx.x * blockDim.x + threadIdx.x,
+                                                 stage[threadIdx.x >> 5]);
+    } else if constexpr (MON) {
         MonAcc m;
         coupled_cell<T, QT, POROUS, true, WIDE>(a, a.c_first + blockIdx.x * blockDim.x + threadIdx.x, &m);
         monitor_block_reduce(m, a.mon + (size_t)blockIdx.x * kMonN);
@@ -1446,6 +1751,8 @@ __global__ void k_build_flags(uint32_t* __restrict__ cellw, const uint32_t* __re
     if (y == 0 || y == ny - 1 || z == 0 || z == nz - 1) w |= kFaceYZ;
     if (x == 0) w |= kXLo;
     if (x == nx - 1) w |= kXHi;
+    if (x == 1) w |= kXLo1;
+    if (x == nx - 2) w |= kXHi1;
     cellw[c] = w;
 }
 

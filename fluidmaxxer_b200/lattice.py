@@ -49,6 +49,7 @@ class CoupledLattice:
         self.shape = (nx, ny, nz)
         self.n = nx * ny * nz
         self.precision = precision
+        self.boundaries = 0   # boundaries added so far
 
     # -- lifetime ------------------------------------------------------------
     def close(self):
@@ -116,30 +117,37 @@ class CoupledLattice:
     def add_ns_velocity_eq(self, mask, ux, uy=0.0, uz=0.0):
         m = _u8(mask, self.n)
         check(self._lib.fm_add_ns_velocity_eq(self.h, m.ctypes.data, m.size, ux, uy, uz))
+        self.boundaries += 1
 
     def add_ns_velocity_neq(self, mask, ux, uy=0.0, uz=0.0):
         m = _u8(mask, self.n)
         check(self._lib.fm_add_ns_velocity_neq(self.h, m.ctypes.data, m.size, ux, uy, uz))
+        self.boundaries += 1
 
     def add_ns_pressure(self, mask, rho_out):
         m = _u8(mask, self.n)
         check(self._lib.fm_add_ns_pressure(self.h, m.ctypes.data, m.size, rho_out))
+        self.boundaries += 1
 
     def add_ns_bounceback(self, mask):
         m = _u8(mask, self.n)
         check(self._lib.fm_add_ns_bounceback(self.h, m.ctypes.data, m.size))
+        self.boundaries += 1
 
     def add_ad_dirichlet(self, mask, phi):
         m = _u8(mask, self.n)
         check(self._lib.fm_add_ad_dirichlet(self.h, m.ctypes.data, m.size, phi))
+        self.boundaries += 1
 
     def add_ad_tanh_pulse(self, mask, phi_base, phi_amp, t_on, t_off, k):
         m = _u8(mask, self.n)
         check(self._lib.fm_add_ad_tanh_pulse(self.h, m.ctypes.data, m.size, phi_base, phi_amp, int(t_on), int(t_off), k))
+        self.boundaries += 1
 
     def add_ad_neumann(self, mask):
         m = _u8(mask, self.n)
         check(self._lib.fm_add_ad_neumann(self.h, m.ctypes.data, m.size))
+        self.boundaries += 1
 
     # -- stepping --------------------------------------------------------------
     def init_equilibrium(self):

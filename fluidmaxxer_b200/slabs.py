@@ -127,11 +127,11 @@ def interior_outlet(slab: Slab) -> np.ndarray:
 
 def split_capable(L) -> bool:
     """A slab lattice can step its planes in parts (fm_step_planes) when its
-    step is one launch and nx * ny is a multiple of 64; otherwise it steps
-    whole (ghost planes included, their updates unread) and the halo moves
-    after the step."""
+    step is one launch, nx * ny is a multiple of 64 and nx is even or no
+    boundary is set; otherwise it steps whole (ghost planes included, their
+    updates unread) and the halo moves after the step."""
     nx, ny, _ = L.shape
-    return L.launches_per_step() == 1 and (nx * ny) % 64 == 0
+    return L.launches_per_step() == 1 and (nx * ny) % 64 == 0 and (nx % 2 == 0 or not L.boundaries)
 
 
 def _neighbours(n: int, index: int, ring: bool):

@@ -406,10 +406,12 @@ int fm_step_status(fm_lattice* lat, int* status);
 
 /* ---- tuning ------------------------------------------------------------------
  * L2 prefetch distance of the fused step kernel, in 256-cell blocks
- * (0 disables the prefetch; negative restores the automatic choice: about
- * half a resident wave for FM_F32, none for FM_F64 and the 16-bit forms, for
- * which a prefetch measured slower on large lattices).  No reference
- * counterpart. */
+ * (0 disables the prefetch; negative restores the automatic choice).  The step
+ * with direct boundary planes fetches its flag words ahead, a quarter of a
+ * resident wave in every form; monitored steps and lattices without direct
+ * planes fetch all they read, half a wave ahead for FM_F32 and not at all for
+ * FM_F64 and the 16-bit forms, for which that measured slower on large
+ * lattices.  No reference counterpart. */
 int fm_set_prefetch_distance(fm_lattice* lat, int blocks);
 
 /* ---- introspection (bench / tests) ---------------------------------------- */
