@@ -146,6 +146,7 @@ struct fm_lattice {
     uint32_t* cellw = nullptr;          // per-cell flag words (k_build_flags)
     bool dirty = true;                  // flags / fusion need rebuilding
     bool split_open = false;            // a step begun by fm_step_planes, not yet finished
+    bool rest = false;                  // both buffers hold every obstacle off the x-faces at the rest equilibrium
     bool chain = false;                 // within fm_step: the last queued work is a step kernel the next one may chain to
     int fuse_outlet = 0, fuse_neumann = 0, fuse_dirichlet = 0;
     uint32_t pf_dist = 0;               // L2 prefetch distance of the fused kernel (blocks)
@@ -527,6 +528,10 @@ int prepare(fm_lattice* L)
         FM_CUDA(cudaMemcpyAsync(L->defer, bits.data(), bits.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, L->stream));
         FM_CUDA(cudaStreamSynchronize(L->stream));
     }
+    // obstacles leave the rest state where a boundary over a cell list may write
+    // them or the porous collision moves them
+    if (L->collision != FM_COLL_BGK || (!L->ns_pre.empty() && !L->fuse_inlet) || (!L->ns_post.empty() && !L->fuse_outlet))
+        L->rest = false;
     if (!L->cellw) {
         rc = dev_alloc(&L->cellw, (size_t)L->ns, L->stream);
         if (rc) return rc;
@@ -535,7 +540,7 @@ int prepare(fm_lattice* L)
         L->cellw, L->solid, L->isotherm != FM_ISO_NONE ? L->region : nullptr, L->ndeferred ? L->defer : nullptr, L->n,
         L->p.nx, L->p.ny, L->p.nz, L->p.periodic_x != 0, L->p.periodic_y != 0, L->p.periodic_z != 0,
         fm::fastdiv_magic((uint32_t)L->p.nx), fm::fastdiv_magic((uint32_t)(L->p.nx * L->p.ny)),
-        L->collision == FM_COLL_BGK);
+        L->collision == FM_COLL_BGK, L->rest && L->elt >= 4 ? (int)(32 / L->elt) : 0, (int)(32 / L->relt));
     FM_CHECK_LAUNCH("k_build_flags");
     if (!L->pf_set) {
         // Direct planes: the flag words a quarter of a resident wave ahead, for
@@ -609,7 +614,8 @@ fm::StepArgs<T, QT> make_args(const fm_lattice* L)
     a.neg_zero = (typename fm::Pop<T>::R)-0.0;
     a.status = L->d_status;
     a.st_rows = 0;
-    a.outputs = 1;
+    a.outputs = fm::kOutX0 | fm::kOutC;
+    a.rest = fm::kRest;
     return a;
 }
 
@@ -815,7 +821,8 @@ int launch_step(fm_lattice* L, bool last)
     }
     // the fused NS + coupling + LDF + AD step
     fm::StepArgs<T, QT> a = make_args<T, QT>(L);
-    a.outputs = last;
+    const bool sampled = L->nprobe && L->probe_every > 0 && s % L->probe_every == 0;
+    a.outputs = (last ? fm::kOutX0 : 0) | (last || sampled ? fm::kOutC : 0);
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     if (L->profiling) {
         if (L->prof_used + 2 > L->prof_ev.size()) {
@@ -1219,6 +1226,14 @@ int ensure_layout(fm_lattice* L)
     return dispatch<LayoutOp>(L, want);
 }
 
+// Populations of f[cur] or f[1-cur], or the obstacles themselves, changed from
+// outside the step: obstacles may not be at rest any more.
+void rest_unknown(fm_lattice* L)
+{
+    if (L->rest) L->dirty = true;
+    L->rest = false;
+}
+
 // One launch per step with every boundary plane a form the batches, the step
 // monitor, the adjoint and the split steps know: for odd nx (whose planes only
 // the direct planes fuse) none of them.
@@ -1366,6 +1381,7 @@ int fm_set_obstacle_mask(fm_lattice* L, const uint8_t* mask, size_t n)
 {
     if (check_mask(L, mask, n, "NSLattice::setObstacleMask:")) return FM_ERR_ARG;
     std::vector<uint32_t> bits = pack_bits(mask, n, L->nwords);
+    if (L->step > 0 || L->split_open) rest_unknown(L);
     FM_CUDA(cudaMemcpyAsync(L->solid, bits.data(), bits.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, L->stream));
     FM_CUDA(cudaStreamSynchronize(L->stream));
     L->dirty = true;
@@ -1380,6 +1396,7 @@ int fm_set_obstacle_bits(fm_lattice* L, const uint32_t* bits, size_t nwords)
     std::memcpy(b.data(), bits, nwords * sizeof(uint32_t));
     const size_t tail = (size_t)L->n & 31;   // clear bits past the last cell
     if (tail) b[(size_t)L->n >> 5] &= (1u << tail) - 1u;
+    if (L->step > 0 || L->split_open) rest_unknown(L);
     FM_CUDA(cudaMemcpyAsync(L->solid, b.data(), b.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, L->stream));
     FM_CUDA(cudaStreamSynchronize(L->stream));
     L->dirty = true;
@@ -1630,6 +1647,11 @@ int fm_init_equilibrium(fm_lattice* L)
     L->mon_steps.clear();
     int rc = dispatch<InitOp>(L);
     if (rc) return rc;
+    // every cell of both buffers is at rest; a density for which j = 0 times
+    // 1 / rho is 0
+    const bool rest = L->collision == FM_COLL_BGK && L->p.rho0 > 1e-30 && L->p.rho0 < 1e30;
+    if (rest != L->rest) L->dirty = true;
+    L->rest = rest;
     L->initialised = true;
     if (L->nprobe && L->probe_every > 0) return take_sample(L);
     return FM_OK;
@@ -1909,6 +1931,7 @@ int fm_set_state(fm_lattice* L, const double* f, const double* g, const double* 
 {
     if (check_lattice(L)) return FM_ERR_ARG;
     if (!L->initialised) return fail(FM_ERR_STATE, "fm_set_state: fm_init_equilibrium not called");
+    if (f) rest_unknown(L);
     int rc = dispatch<SetPops>(L, f, g);
     if (!rc && f) L->inlet_state = 0;   // every population, x = 0 included, is the caller's
     if (rc) return rc;
@@ -1991,6 +2014,7 @@ int pull_copy_run(fm_lattice* L, int reps, double* ms_per_rep, double* bytes_per
     if (c_hi <= c_lo || (L->layout == 1 && c_hi <= c_lo + 2))
         return fail(FM_ERR_ARG, "fm_bench_pull_copy: lattice too small (needs more than two z-planes)");
     const int A = L->cur, B = 1 - L->cur;
+    rest_unknown(L);   // the copy scrambles f[B]
     // the pair layout: whole words, every source off the fold points
     const long long h = nx / 2, hny = h * L->p.ny;
     const long long w_lo = hny + h + 1, w_hi = (long long)L->n / 2 - hny - h - 1;
@@ -2221,9 +2245,9 @@ int batch_upload_const(fm_batch* B)
     return FM_OK;
 }
 
-// `last`: the batch's outputs may be read before its next step
+// `outputs`: what may be read before the next step (StepArgs::outputs)
 template <typename T, typename QT>
-int batch_launch_step(fm_batch* B, int parity, bool last)
+int batch_launch_step(fm_batch* B, int parity, int outputs)
 {
     if (B->mode == 3) {
         const auto* args = reinterpret_cast<const fm::StepArgs<T, QT>*>(B->h_args[parity].data());
@@ -2233,7 +2257,7 @@ int batch_launch_step(fm_batch* B, int parity, bool last)
         for (size_t i = 0; i < B->lats.size(); ++i) {
             const int k = B->side_of[i];
             fm::StepArgs<T, QT> a = args[i];
-            a.outputs = last;
+            a.outputs = outputs;
             const int grid = grid_for(B->lats[i]->n);
             if (B->collision == FM_COLL_BGK) launch_coupled<T, QT, false, false>(B->lats[i], grid, B->side[k], a, chain[k]);
             else launch_coupled<T, QT, true, false>(B->lats[i], grid, B->side[k], a, chain[k]);
@@ -2269,7 +2293,10 @@ template <typename T, typename QT> struct BatchConstOp {
     static int run(fm_lattice*, fm_batch* B) { return batch_upload_const<T, QT>(B); }
 };
 template <typename T, typename QT> struct BatchStepOp {
-    static int run(fm_lattice*, fm_batch* B, int parity, bool last) { return batch_launch_step<T, QT>(B, parity, last); }
+    static int run(fm_lattice*, fm_batch* B, int parity, int outputs)
+    {
+        return batch_launch_step<T, QT>(B, parity, outputs);
+    }
 };
 
 template <typename T, typename QT>
@@ -2297,7 +2324,10 @@ template <typename T, typename QT> struct BatchGridOp {
 
 int batch_dispatch_items(fm_batch* B) { return dispatch<BatchItemsOp>(B->lats[0], B); }
 int batch_dispatch_grid(fm_batch* B) { return dispatch<BatchGridOp>(B->lats[0], B); }
-int batch_dispatch_step(fm_batch* B, int parity, bool last) { return dispatch<BatchStepOp>(B->lats[0], B, parity, last); }
+int batch_dispatch_step(fm_batch* B, int parity, int outputs)
+{
+    return dispatch<BatchStepOp>(B->lats[0], B, parity, outputs);
+}
 int batch_dispatch_const(fm_batch* B)
 {
     return (B->mode == 1 || B->mode == 2) ? dispatch<BatchConstOp>(B->lats[0], B) : FM_OK;
@@ -2384,9 +2414,10 @@ int batch_launch_probes(fm_batch* B)
 // one step of every lattice; `s` is the step number being completed
 int batch_one(fm_batch* B, long long s, int parity, bool last)
 {
-    int rc = batch_dispatch_step(B, parity, last);
+    const bool sampled = B->probe_every > 0 && s % B->probe_every == 0;
+    int rc = batch_dispatch_step(B, parity, (last ? fm::kOutX0 : 0) | (last || sampled ? fm::kOutC : 0));
     if (rc) return rc;
-    if (B->probe_every > 0 && s % B->probe_every == 0) return batch_launch_probes(B);
+    if (sampled) return batch_launch_probes(B);
     return FM_OK;
 }
 
@@ -2666,10 +2697,10 @@ int fm_batch_autotune(fm_batch* B, int trial_steps, int* mode, int* block, int* 
                 if (!rc) rc = batch_dispatch_const(B);
                 if (rc) break;
                 int parity = B->lats[0]->cur;
-                for (int i = 0; i < 2 && !rc; ++i, parity ^= 1) rc = batch_dispatch_step(B, parity, true);
+                for (int i = 0; i < 2 && !rc; ++i, parity ^= 1) rc = batch_dispatch_step(B, parity, fm::kOutX0 | fm::kOutC);
                 if (rc) break;
                 cudaEventRecord(e0, B->stream);
-                for (int i = 0; i < trials && !rc; ++i, parity ^= 1) rc = batch_dispatch_step(B, parity, true);
+                for (int i = 0; i < trials && !rc; ++i, parity ^= 1) rc = batch_dispatch_step(B, parity, fm::kOutX0 | fm::kOutC);
                 cudaEventRecord(e1, B->stream);
                 if (cudaEventSynchronize(e1) != cudaSuccess) { rc = fail(FM_ERR_CUDA, "autotune sync failed"); break; }
                 float ms = 0.0f;
@@ -2777,7 +2808,10 @@ int adj_forward(AdjCtx& X, const AdjState& in, AdjState& out)
     a.fB = (T*)out.f; a.gB = (T*)out.g;
     a.phi = (R*)out.phi; a.q = (QT*)out.q;
     a.x0post = (T*)X.x0scratch;
-    a.outputs = 0;   // the recomputed states are read in the fused representation only
+    // the recomputed states are read in the fused representation, their C in the
+    // region; their buffers held other states' obstacles
+    a.outputs = 0;
+    a.rest = 0u;
     ++X.forward_steps;
     if (L->collision == FM_COLL_BGK) launch_coupled<T, QT, false, false>(L, grid_for(L->n), L->stream, a);
     else launch_coupled<T, QT, true, false>(L, grid_for(L->n), L->stream, a);
@@ -3111,6 +3145,7 @@ static int zplane_copy(fm_lattice* L, int z, void* buf, int pack)
     if (check_lattice(L)) return FM_ERR_ARG;
     if (!buf || z < 0 || z >= L->p.nz) return fail(FM_ERR_ARG, "fm_pack/unpack_zplane: z outside [0, nz) or null buffer");
     if (!L->initialised) return fail(FM_ERR_STATE, "fm_pack/unpack_zplane: lattice not initialised");
+    if (!pack) rest_unknown(L);
     const long long nxy = (long long)L->p.nx * L->p.ny;
     const int grid = grid_for(26LL * nxy);
     void* f = L->f[L->cur];
@@ -3156,6 +3191,7 @@ static int zhalo_copy(fm_lattice* L, int z, int dir, void* buf, int pack)
     if (!buf || z < 0 || z >= L->p.nz || (dir != 1 && dir != -1))
         return fail(FM_ERR_ARG, "fm_pack/unpack_zhalo: z outside [0, nz), dir not +1 / -1, or null buffer");
     if (!L->initialised) return fail(FM_ERR_STATE, "fm_pack/unpack_zhalo: lattice not initialised");
+    if (!pack) rest_unknown(L);
     const long long nxy = (long long)L->p.nx * L->p.ny;
     const int grid = grid_for(6LL * nxy);
     const int b = L->split_open ? 1 - L->cur : L->cur;
