@@ -568,8 +568,8 @@ fm::StepArgs<T, QT> make_args(const fm_lattice* L)
     a.fB = (T*)L->f[B];
     a.gA = (const T*)L->g[A];
     a.gB = (T*)L->g[B];
-    a.phi = (R*)L->phi;
-    a.q = (QT*)L->q;
+    a.phi = a.phi_out = (R*)L->phi;
+    a.q = a.q_out = (QT*)L->q;
     a.cellw = L->cellw;
     a.porosity = (const R*)L->por;
     a.tau_ad = L->tau_field ? (const R*)L->tau : nullptr;
@@ -2762,9 +2762,12 @@ struct AdjCtx {
     long long forward_steps = 0;   // recomputed forward steps (statistics)
     void* x0scratch = nullptr;     // x0post of recomputed steps
     AdjState lam[2];               // adjoint state (R): f 19, g 7, phi, q
-    void *lfi = nullptr, *lgi = nullptr;
+    // (lam[i].f, .g: the adjoints of the populations the step pulled, AdjArgs::lfi / lgi)
+    void* x1 = nullptr;            // f at x = 1 of the state last stepped back from [19][rows_stride]
     double *gpor = nullptr, *gpar = nullptr;
     int cur = 0;
+    bool first = true;             // no backward step yet
+    bool chain = false;            // the last work queued is a kernel the next one may chain to
 };
 
 // bump allocator over the lattice's adjoint arena (256-byte aligned pieces)
@@ -2801,25 +2804,26 @@ int adj_forward(AdjCtx& X, const AdjState& in, AdjState& out)
 {
     using R = typename fm::Pop<T>::R;
     fm_lattice* L = X.L;
-    FM_CUDA(cudaMemcpyAsync(out.phi, in.phi, (size_t)L->ns * sizeof(R), cudaMemcpyDeviceToDevice, L->stream));
-    FM_CUDA(cudaMemcpyAsync(out.q, in.q, (size_t)L->ns * sizeof(QT), cudaMemcpyDeviceToDevice, L->stream));
     fm::StepArgs<T, QT> a = make_args<T, QT>(L);
     a.fA = (const T*)in.f; a.gA = (const T*)in.g;
     a.fB = (T*)out.f; a.gB = (T*)out.g;
-    a.phi = (R*)out.phi; a.q = (QT*)out.q;
+    // C and q of a recomputed state are read, and so written, in the region only
+    a.phi = (const R*)in.phi; a.q = (const QT*)in.q;
+    a.phi_out = (R*)out.phi; a.q_out = (QT*)out.q;
     a.x0post = (T*)X.x0scratch;
     // the recomputed states are read in the fused representation, their C in the
     // region; their buffers held other states' obstacles
     a.outputs = 0;
     a.rest = 0u;
     ++X.forward_steps;
-    if (L->collision == FM_COLL_BGK) launch_coupled<T, QT, false, false>(L, grid_for(L->n), L->stream, a);
-    else launch_coupled<T, QT, true, false>(L, grid_for(L->n), L->stream, a);
+    if (L->collision == FM_COLL_BGK) launch_coupled<T, QT, false, false>(L, grid_for(L->n), L->stream, a, X.chain);
+    else launch_coupled<T, QT, true, false>(L, grid_for(L->n), L->stream, a, X.chain);
     FM_CHECK_LAUNCH("adjoint forward");
+    X.chain = true;
     return FM_OK;
 }
 
-// backward step t (forward step t maps X_{t-1} -> X_t): lam[cur] = lambda_t -> lambda_{t-1}
+// backward step t (forward step t maps X_{t-1} -> X_t): lam[cur] of step t+1 -> lam[1-cur] of step t
 template <typename T, typename QT>
 int adj_backward(AdjCtx& X, long long t, const AdjState& xprev)
 {
@@ -2829,26 +2833,33 @@ int adj_backward(AdjCtx& X, long long t, const AdjState& xprev)
     A.a = make_args<T, QT>(L);
     A.a.fA = (const T*)xprev.f; A.a.gA = (const T*)xprev.g;
     A.a.fB = nullptr; A.a.gB = nullptr;
-    A.a.phi = (R*)xprev.phi; A.a.q = (QT*)xprev.q;
-    A.a.pf_dist = 0;
+    A.a.phi = (const R*)xprev.phi; A.a.q = (const QT*)xprev.q;
+    A.a.phi_out = nullptr; A.a.q_out = nullptr;
     AdjState& l1 = X.lam[X.cur];
     AdjState& l0 = X.lam[1 - X.cur];
-    A.lf1 = (const R*)l1.f; A.lg1 = (const R*)l1.g; A.lphi1 = (const R*)l1.phi; A.lq1 = (const R*)l1.q;
-    A.lfi = (R*)X.lfi; A.lgi = (R*)X.lgi;
+    A.lfi1 = (const R*)l1.f; A.lgi1 = (const R*)l1.g; A.lphi1 = (const R*)l1.phi; A.lq1 = (const R*)l1.q;
+    A.lfi = (R*)l0.f; A.lgi = (R*)l0.g;
     A.lphi0 = (R*)l0.phi; A.lq0 = (R*)l0.q;
+    A.x1 = (R*)X.x1;
     A.gpor = X.gpor; A.gpar = X.gpar;
     A.wl = (R)X.wl[(size_t)(t - X.s0)];
-    if (L->collision == FM_COLL_BGK) {
-        fm::k_adj_cell<T, QT, false><<<grid_for(L->n), kBlock, 0, L->stream>>>(A);
-        fm::k_adj_stream<T, QT, false><<<grid_for(L->n), kBlock, 0, L->stream>>>(A, (R*)l0.f, (R*)l0.g);
-    } else {
-        fm::k_adj_cell<T, QT, true><<<grid_for(L->n), kBlock, 0, L->stream>>>(A);
-        fm::k_adj_stream<T, QT, true><<<grid_for(L->n), kBlock, 0, L->stream>>>(A, (R*)l0.f, (R*)l0.g);
-    }
-    if (L->fuse_inlet)
-        fm::k_adj_inlet<T, QT><<<grid_for((long long)L->p.ny * L->p.nz * 32), kBlock, 0, L->stream>>>(A, (R*)l0.f);
+    A.first = X.first;
+    // a step kernel or a backward step before it ends first (pdl_wait)
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid_for(L->n, fm::kAdjThreads));
+    cfg.blockDim = dim3(fm::kAdjThreads);
+    cfg.stream = L->stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = X.chain ? 1 : 0;
+    if (L->collision == FM_COLL_BGK) cudaLaunchKernelEx(&cfg, fm::k_adj_step<T, QT, false>, A);
+    else cudaLaunchKernelEx(&cfg, fm::k_adj_step<T, QT, true>, A);
     FM_CHECK_LAUNCH("adjoint step");
     X.cur = 1 - X.cur;
+    X.first = false;
+    X.chain = true;
     return FM_OK;
 }
 
@@ -2960,6 +2971,7 @@ int adjoint_run(fm_lattice* L, int nsteps, const double* target, int ntarget, in
     X.every = L->probe_every;
     const int C = checkpoint_every > 0 ? std::min(checkpoint_every, nsteps) : nsteps;
     const int nseg = (nsteps + C - 1) / C;
+    const size_t nwarps = (size_t)grid_for(L->n, fm::kAdjThreads) * (fm::kAdjThreads / 32);   // of a k_adj_step launch
     const int nstates = std::max(1, std::min(max_states > 0 ? max_states : C - 1, C - 1));
     std::vector<AdjState> snaps((size_t)nseg);
     // ---- workspace: one arena, carved (a dry run sizes it) ----
@@ -2970,10 +2982,9 @@ int adjoint_run(fm_lattice* L, int nsteps, const double* target, int ntarget, in
         for (auto& st : X.pool) cv.state(L, st, L->elt, L->elt, L->relt, L->qelt);
         cv.state(L, X.lam[0], sizeof(R), sizeof(R), sizeof(R), sizeof(R));
         cv.state(L, X.lam[1], sizeof(R), sizeof(R), sizeof(R), sizeof(R));
-        X.lfi = cv.take((size_t)19 * L->ns * sizeof(R));
-        X.lgi = cv.take((size_t)7 * L->ns * sizeof(R));
+        X.x1 = L->rows_stride ? cv.take((size_t)19 * L->rows_stride * sizeof(R)) : nullptr;
         X.gpor = (double*)cv.take(sizeof(double) * L->ns);
-        X.gpar = (double*)cv.take(sizeof(double) * 3);
+        X.gpar = (double*)cv.take(sizeof(double) * 3 * (nwarps + 1));   // and the folded sums
         X.x0scratch = L->rows_stride ? cv.take((size_t)19 * L->rows_stride * L->elt) : nullptr;
     };
     Carver dry;
@@ -3022,7 +3033,8 @@ int adjoint_run(fm_lattice* L, int nsteps, const double* target, int ntarget, in
         FM_CUDA(cudaMemsetAsync(X.lam[i].q, 0, (size_t)L->ns * sizeof(R), L->stream));
     }
     FM_CUDA(cudaMemsetAsync(X.gpor, 0, sizeof(double) * L->ns, L->stream));
-    FM_CUDA(cudaMemsetAsync(X.gpar, 0, sizeof(double) * 3, L->stream));
+    FM_CUDA(cudaMemsetAsync(X.gpar, 0, sizeof(double) * 3 * (nwarps + 1), L->stream));
+    if (X.x1) FM_CUDA(cudaMemsetAsync(X.x1, 0, (size_t)19 * L->rows_stride * sizeof(R), L->stream));
     for (int k = nseg - 1; k >= 0 && !rc; --k) {
         const long long a = X.s0 + (long long)k * C;
         const long long b = std::min(a + C, X.s0 + nsteps);
@@ -3030,7 +3042,9 @@ int adjoint_run(fm_lattice* L, int nsteps, const double* target, int ntarget, in
     }
     if (rc) return rc;
     double gp[3] = {0, 0, 0};
-    FM_CUDA(cudaMemcpyAsync(gp, X.gpar, sizeof(gp), cudaMemcpyDeviceToHost, L->stream));
+    fm::k_adj_fold<<<1, 1024, 0, L->stream>>>(X.gpar, (int)nwarps, X.gpar + 3 * nwarps);
+    FM_CHECK_LAUNCH("k_adj_fold");
+    FM_CUDA(cudaMemcpyAsync(gp, X.gpar + 3 * nwarps, sizeof(gp), cudaMemcpyDeviceToHost, L->stream));
     if (grad_porosity)
         FM_CUDA(cudaMemcpyAsync(grad_porosity, X.gpor, sizeof(double) * L->n, cudaMemcpyDeviceToHost, L->stream));
     FM_CUDA(cudaStreamSynchronize(L->stream));

@@ -4,19 +4,23 @@
 // phi_s is the AD scalar computed during step s (the LDF source of step s+1
 // reads it).  f_s is held as the fused kernel holds it: at x = 0 the
 // VelocityDirichletNEQ values the next pull reads, derived from f_s at x = 1.
-// Given the adjoint lambda_{s+1} = dL/dX_{s+1}, two kernels produce lambda_s:
+// Given the adjoint lambda_{s+1} = dL/dX_{s+1}, one kernel produces lambda_s:
 //
-//   k_adj_cell    per cell: recompute the forward step at the cell (the same
-//                 device functions as k_coupled_step), then apply in reverse
-//                 the AD boundaries, the D3Q7 collision, the LDF source, the
-//                 coupling velocity, the pressure outlet and the NS collision.
-//                 Writes the adjoints of the pulled populations (lfi, lgi),
-//                 lambda(phi_s), lambda(q_s) and accumulates the gradients of
-//                 the isotherm parameters and of the porosity field.
-//   k_adj_stream  per cell: the transposed pull (a gather of lfi / lgi from
-//                 the cells that read each population: neighbour pull,
-//                 keep-local, own-opposite bounce-back, obstacle reversal);
-//   k_adj_inlet   per inlet row: the NEQ inlet's adjoint from x = 0 into x = 1.
+//   k_adj_step  per cell: gather lambda f_{s+1} and lambda g_{s+1} by the
+//               transposed pull from the adjoints of the pulled populations
+//               the backward step before left (each population was read by the
+//               cells that pulled it: neighbour pull, keep-local, own-opposite
+//               bounce-back, obstacle reversal), move the NEQ inlet's adjoint
+//               from x = 0 into x = 1, recompute the forward step at the cell
+//               (the same arithmetic as k_coupled_step), then apply in reverse
+//               the AD boundaries, the D3Q7 collision, the LDF source, the
+//               coupling velocity, the pressure outlet and the NS collision.
+//               Writes the adjoints of the populations this step pulled (lfi,
+//               lgi), lambda(phi_s), lambda(q_s) and accumulates the gradients
+//               of the isotherm parameters and of the porosity field.
+//
+// The adjoint state therefore travels as (lfi, lgi): a gather at the start of
+// the next step takes the place of a pass of its own over all 26 planes.
 //
 // Non-smooth points take the derivative of the branch the forward took (the
 // phi clamp, max(c, eps), the porosity clamp).  Supported set-up: BGK or
@@ -34,60 +38,177 @@ template <typename T, typename QT>
 struct AdjArgs {
     using R = typename Pop<T>::R;
     StepArgs<T, QT> a;              // forward step from X_s (fA = f_s, gA = g_s, phi = phi_s, q = q_s)
-    const R* __restrict__ lf1;      // lambda f_{s+1}   [19][ns]
-    const R* __restrict__ lg1;      // lambda g_{s+1}   [7][ns]
+    const R* __restrict__ lfi1;     // adjoints of the D3Q19 populations step s+2 pulled [19][ns]
+    const R* __restrict__ lgi1;     // the same of the D3Q7 populations [7][ns]
     const R* __restrict__ lphi1;    // lambda phi_{s+1}
     const R* __restrict__ lq1;      // lambda q_{s+1}
-    R* __restrict__ lfi;            // out: lambda of the pulled D3Q19 populations
-    R* __restrict__ lgi;            // out: lambda of the pulled D3Q7 populations
+    R* __restrict__ lfi;            // out: adjoints of the D3Q19 populations step s+1 pulls
+    R* __restrict__ lgi;            // out: the same of the D3Q7 populations
     R* __restrict__ lphi0;          // out: lambda phi_s
     R* __restrict__ lq0;            // out: lambda q_s
+    R* __restrict__ x1;             // [19][rows]: f_{s+1} at x = 1 in, f_s at x = 1 out
     double* __restrict__ gpor;      // += dL/d porosity per cell (porous collision)
-    double* __restrict__ gpar;      // += dL/d (isotherm a, b, k)
+    double* __restrict__ gpar;      // += dL/d (isotherm a, b, k), per warp [warps][3]
     R wl;                           // loss weight on phi_{s+1} of the outlet plane (0: not sampled)
+    int first;                      // no backward step before: lfi1, lgi1 are zero
 };
 
-// d feq_k / du of the second-order equilibrium: w rho (3 c + 9 (c.u) c - 3 u)
-template <typename R>
-__device__ __forceinline__ void dfeq_du(int k, R w, R rho, R ux, R uy, R uz, R& gx, R& gy, R& gz)
+// c v for a velocity component c of direction K (v, 0 or -v)
+template <int C, typename R>
+__device__ __forceinline__ R times_c(R v)
 {
-    const R cx = (R)cx19(k), cy = (R)cy19(k), cz = (R)cz19(k);
-    const R e = cx * ux + cy * uy + cz * uz;
-    gx = w * rho * (R(3) * cx + R(9) * e * cx - R(3) * ux);
-    gy = w * rho * (R(3) * cy + R(9) * e * cy - R(3) * uy);
-    gz = w * rho * (R(3) * cz + R(9) * e * cz - R(3) * uz);
+    return C == 0 ? R(0) : (C > 0 ? v : -v);
+}
+
+// d feq_K / du of the second-order equilibrium: w rho (3 c + 9 (c.u) c - 3 u)
+template <int K, typename R>
+__device__ __forceinline__ void dfeq_du(R rho, R ux, R uy, R uz, R& gx, R& gy, R& gz)
+{
+    const R e9 = R(9) * cdot<cx19(K), cy19(K), cz19(K)>(ux, uy, uz);
+    const R wr = w19<R>(K) * rho;
+    gx = wr * ((R(3 * cx19(K)) + times_c<cx19(K)>(e9)) - R(3) * ux);
+    gy = wr * ((R(3 * cy19(K)) + times_c<cy19(K)>(e9)) - R(3) * uy);
+    gz = wr * ((R(3 * cz19(K)) + times_c<cz19(K)>(e9)) - R(3) * uz);
+}
+
+// feq_K / (w_K rho), m = 1.5 u^2
+template <int K, typename R>
+__device__ __forceinline__ R poly19(R ux, R uy, R uz, R m)
+{
+    const R e = cdot<cx19(K), cy19(K), cz19(K)>(ux, uy, uz);
+    return R(1) + R(3) * e + R(4.5) * e * e - m;
+}
+
+// f(std::integral_constant<int, K>) for K = 0..18
+template <typename F, int... Ks>
+__device__ __forceinline__ void each19(F f, std::integer_sequence<int, Ks...>)
+{
+    (f(std::integral_constant<int, Ks>{}), ...);
 }
 
 template <typename R>
-__device__ __forceinline__ R poly19(int k, R ux, R uy, R uz)
+__device__ __forceinline__ R warp_sum_r(R v)
 {
-    const R e = (R)cx19(k) * ux + (R)cy19(k) * uy + (R)cz19(k) * uz;
-    return R(1) + R(3) * e + R(4.5) * e * e - R(1.5) * (ux * ux + uy * uy + uz * uz);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
 }
 
-// resident 256-thread blocks per SM k_adj_cell is compiled for (FP64 needs its
-// registers: the recomputed forward and the adjoint are both live)
+// The transposed pull of direction J at a cell away from the y/z faces: the
+// sum of the adjoints of the pulls that read the cell's population J -- by the
+// cell at c + c_J, by the cell itself where that lies outside (keep-local), by
+// its own opposite direction (a link to an obstacle at c + c_J, or an obstacle
+// cell, whose bits lk 1..18 are all set).
+template <int J, bool BB, typename R>
+__device__ __forceinline__ R gather19_fast(const R* __restrict__ base, uint32_t ns, int nx, int nxy, int px, bool xlo,
+                                           bool xhi, uint32_t lk, bool solid)
+{
+    constexpr int CX = cx19(J), CY = cy19(J), CZ = cz19(J), O = opp19(J);
+    if (J == 0) return base[0];
+    const bool own = BB && ((lk >> O) & 1u);
+    const bool out = CX != 0 && (CX > 0 ? xhi : xlo);    // c + c_J beyond an x-face
+    const bool keep = CX != 0 && (CX > 0 ? xlo : xhi);   // c - c_J beyond an x-face: the cell kept its own value
+    uint32_t off = (uint32_t)J * ns + (uint32_t)(CX + CY * nx + CZ * nxy);
+    if (out) off -= (uint32_t)(CX * nx);                 // periodic x
+    if (own) off = (uint32_t)O * ns;
+    R v = (out && !px && !own) ? R(0) : base[off];
+    if (keep && !px && !solid) v += base[(uint32_t)J * ns];
+    return v;
+}
+// the same for any cell
+template <int J, bool BB, typename R>
+__device__ __forceinline__ R gather19(const R* __restrict__ l, uint32_t ns, uint32_t c, const Nbr& nb, uint32_t w,
+                                      bool solid)
+{
+    constexpr int CX = cx19(J), CY = cy19(J), CZ = cz19(J), O = opp19(J);
+    if (J == 0) return l[c];
+    const bool in_o = nb.inside<-CX, -CY, -CZ>(), in_j = nb.inside<CX, CY, CZ>();
+    const bool link = BB && ((w >> O) & 1u);
+    R v = R(0);
+    if (in_o && !link && !solid) v += l[(uint32_t)J * ns + (uint32_t)nb.src<-CX, -CY, -CZ>()];
+    if (!in_j && !solid) v += l[(uint32_t)J * ns + c];
+    if (solid || (in_o && link)) v += l[(uint32_t)O * ns + c];
+    return v;
+}
+// D3Q7 has no reflection
+template <int J, typename R>
+__device__ __forceinline__ R gather7_fast(const R* __restrict__ base, uint32_t ns, int nx, int nxy, int px, bool xlo,
+                                          bool xhi)
+{
+    return gather19_fast<J, false>(base, ns, nx, nxy, px, xlo, xhi, 0u, false);
+}
+static_assert(cx19(1) == cx7(1) && cx19(2) == cx7(2) && cy19(3) == cy7(3) && cy19(4) == cy7(4) && cz19(5) == cz7(5) &&
+                  cz19(6) == cz7(6),
+              "the D3Q7 directions are the first seven of D3Q19");
+
+// threads per block, and resident blocks per SM k_adj_step is compiled for: 80
+// registers (FP32) and 168 (FP64), the recomputed forward and the adjoint both
+// live.  A gradient of 240 steps at 48x80x80: FP32 6 blocks 19.6 ms, 7 19.8, 8
+// 19.7; FP64 2 blocks 36.4 ms, 3 32.5, 4 31.3 (but 24x40x40 8.1, 7.6, 8.1).
+constexpr int kAdjThreads = 128;
 template <typename T>
-constexpr int kAdjBlocks = sizeof(T) == 8 ? 1 : 3;
+constexpr int kAdjBlocks = sizeof(T) == 8 ? 3 : 6;
 
+// Bound by latency and instruction issue (24 FP32 warps an SM, 2600 instructions
+// each).  It replaces a cell kernel, a stream kernel and an inlet kernel, which
+// passed the 26 adjoint planes through memory once more (564 against 352 B a
+// cell), formed every product with the zero velocity components and took the
+// neighbour table in every warp.  All loads of populations and adjoints come
+// first, so a cell waits for memory once: a gradient of 240 steps at 48x80x80
+// took 26.7 ms with the three kernels, 21.5 with one that loads where it uses,
+// 19.6 with this order (FP64 49.7, 43.8, 32.5).
 template <typename T, typename QT, bool POROUS>
-__global__ void __launch_bounds__(256, kAdjBlocks<T>) k_adj_cell(const AdjArgs<T, QT> A)
+__global__ void __launch_bounds__(kAdjThreads, kAdjBlocks<T>) k_adj_step(const AdjArgs<T, QT> A)
 {
     using R = typename Pop<T>::R;
     const StepArgs<T, QT>& a = A.a;
+    __shared__ R line[kAdjThreads / 32][20];   // one inlet row at a time, per warp
     const uint32_t cg = blockIdx.x * blockDim.x + threadIdx.x;
     const bool active = cg < (uint32_t)a.n;
     const uint32_t c = active ? cg : (uint32_t)a.n - 1u;
-    int x, y, z;
-    cell_xyz(c, a.nx, a.ny, a.div_nx, a.div_nxy, x, y, z);
-    const Nbr nb(x, y, z, a.nx, a.ny, a.nz, a.px, a.py, a.pz);
+    const int lane = threadIdx.x & 31;
     const uint32_t w = __ldg(a.cellw + c);
+    pdl_wait();
     const bool solid = !POROUS && (w & kSolid);
+    const bool xlo = (w & kXLo) != 0u, xhi = (w & kXHi) != 0u;
     const uint32_t ns = a.ns;
+    const int nxy = a.nx * a.ny;
+    const uint32_t lk = solid ? 0x7fffeu : w;
+    const bool face = __any_sync(0xffffffffu, w & kFaceYZ);
+    int x = 1, y = 1, z = 1;
+    if (face) cell_xyz(c, a.nx, a.ny, a.div_nx, a.div_nxy, x, y, z);
+    const Nbr nb(x, y, z, a.nx, a.ny, a.nz, a.px, a.py, a.pz);
 
     // ---- forward recompute of the NS part ----
     R fi[19];
-    pull19_all<T, !POROUS>(fi, a.fA, ns, c, nb, w, a.f_shift, Seq19{});
+    if (face) pull19_all<T, !POROUS>(fi, a.fA, ns, c, nb, w, a.f_shift, Seq19{});
+    else pull19_fast_all<T, !POROUS>(fi, a.fA + c, ns, a.nx, nxy, a.px, xlo, xhi, lk, R(0), Seq19{});
+    R gi[7];
+    if (face) pull7(a, c, nb, gi);
+    else pull7_fast_all<T>(gi, a.gA + c, ns, a.nx, nxy, a.px, xlo, xhi, a.g_shift, Seq7{});
+    R lg[7];
+    if (face) {
+        each19([&](auto k) {
+            constexpr int K = decltype(k)::value;
+            if constexpr (K < 7) lg[K] = gather19<K, false>(A.lgi1, ns, c, nb, 0u, false);
+        }, Seq19{});
+    } else {
+        each19([&](auto k) {
+            constexpr int K = decltype(k)::value;
+            if constexpr (K < 7) lg[K] = gather7_fast<K>(A.lgi1 + c, ns, a.nx, nxy, a.px, xlo, xhi);
+        }, Seq19{});
+    }
+    R lf[19];
+    if (face)
+        each19([&](auto k) {
+            constexpr int K = decltype(k)::value;
+            lf[K] = gather19<K, !POROUS>(A.lfi1, ns, c, nb, w, solid);
+        }, Seq19{});
+    else
+        each19([&](auto k) {
+            constexpr int K = decltype(k)::value;
+            lf[K] = gather19_fast<K, !POROUS>(A.lfi1 + c, ns, a.nx, nxy, a.px, xlo, xhi, lk, solid);
+        }, Seq19{});
     R rho = R(0), ubx = R(0), uby = R(0), ubz = R(0), ux = R(0), uy = R(0), uz = R(0), por = R(1);
     bool por_free = false;   // porosity strictly inside [0,1]: the clamp passes the derivative
     if (!solid) {
@@ -106,36 +227,42 @@ __global__ void __launch_bounds__(256, kAdjBlocks<T>) k_adj_cell(const AdjArgs<T
             ux *= ph; uy *= ph; uz *= ph;
         }
     }
-    // post-collision populations fh (BGK: fi + omega (feq - fi); obstacle: fi)
-    R fh[19];
-#pragma unroll
-    for (int k = 0; k < 19; ++k) {
-        if (solid) { fh[k] = fi[k]; continue; }
-        const R feq = w19<R>(k) * rho * poly19(k, ux, uy, uz);
-        fh[k] = fi[k] + a.omega * (feq - fi[k]);
-    }
-    // moments of fh (the x-1 neighbour's velocity for the outlet)
+    const R m15 = R(1.5) * (ux * ux + uy * uy + uz * uz);
+    // post-collision populations (BGK: fi + omega (feq - fi); obstacle: fi), in place
+    if (!solid)
+        each19([&](auto k) {
+            constexpr int K = decltype(k)::value;
+            const R feq = w19<R>(K) * rho * poly19<K>(ux, uy, uz, m15);
+            fi[K] = fi[K] + a.omega * (feq - fi[K]);
+        }, Seq19{});
+    // their moments (the x-1 neighbour's velocity for the outlet)
     R rh, hx, hy, hz;
-    moments19(fh, rh, hx, hy, hz, Seq19{});
+    moments19(fi, rh, hx, hy, hz, Seq19{});
     const R ih = (rh > R(0)) ? (R(1) / rh) : R(0);
     const R uhx = hx * ih, uhy = hy * ih, uhz = hz * ih;
-    const bool outlet = a.fuse_outlet && x == a.nx - 1;
-    const R uNx = __shfl_up_sync(0xffffffffu, uhx, 1);
-    const R uNy = __shfl_up_sync(0xffffffffu, uhy, 1);
-    const R uNz = __shfl_up_sync(0xffffffffu, uhz, 1);
-    // post-boundary populations and the coupling velocity of them
-    R fp[19];
-#pragma unroll
-    for (int k = 0; k < 19; ++k)
-        fp[k] = outlet ? w19<R>(k) * a.rho_out * poly19(k, uNx, uNy, uNz) : fh[k];
-    R rp, px, py, pz;
-    moments19(fp, rp, px, py, pz, Seq19{});
-    const R ip = (rp > R(0)) ? (R(1) / rp) : R(0);
-    const R uax = a.coupling ? px * ip : R(0), uay = a.coupling ? py * ip : R(0), uaz = a.coupling ? pz * ip : R(0);
+    // the coupling velocity of the populations after the outlet boundary
+    const bool outlet = a.fuse_outlet && xhi;
+    R rp = rh, ip = ih, uax = uhx, uay = uhy, uaz = uhz;
+    R uNx = R(0), uNy = R(0), uNz = R(0);
+    if (__any_sync(0xffffffffu, outlet)) {
+        uNx = __shfl_up_sync(0xffffffffu, uhx, 1);
+        uNy = __shfl_up_sync(0xffffffffu, uhy, 1);
+        uNz = __shfl_up_sync(0xffffffffu, uhz, 1);
+        if (outlet) {
+            R fp[19], jx, jy, jz;
+            const R mN = R(1.5) * (uNx * uNx + uNy * uNy + uNz * uNz);
+            each19([&](auto k) {
+                constexpr int K = decltype(k)::value;
+                fp[K] = w19<R>(K) * a.rho_out * poly19<K>(uNx, uNy, uNz, mN);
+            }, Seq19{});
+            moments19(fp, rp, jx, jy, jz, Seq19{});
+            ip = (rp > R(0)) ? (R(1) / rp) : R(0);
+            uax = jx * ip; uay = jy * ip; uaz = jz * ip;
+        }
+    }
+    if (!a.coupling) uax = uay = uaz = R(0);
 
     // ---- forward recompute of the AD part ----
-    R gi[7];
-    pull7(a, c, nb, gi);
     R gs = gi[0];
 #pragma unroll
     for (int k = 1; k < 7; ++k) gs += gi[k];
@@ -145,23 +272,21 @@ __global__ void __launch_bounds__(256, kAdjBlocks<T>) k_adj_cell(const AdjArgs<T
     const bool region = a.isotherm != 0 && (w & kRegion);
 
     // ---- adjoint of the AD boundaries and collision ----
-    R lg[7];
-#pragma unroll
-    for (int k = 0; k < 7; ++k) lg[k] = A.lg1[(uint32_t)k * ns + c];
-    if (a.fuse_dirichlet && x == 0) {
-#pragma unroll
-        for (int k = 0; k < 7; ++k) lg[k] = R(0);
-    }
-    if (a.fuse_neumann) {
-        if (x == a.nx - 1) {
+    if (__any_sync(0xffffffffu, xlo || xhi)) {
+        if (a.fuse_dirichlet && xlo) {
 #pragma unroll
             for (int k = 0; k < 7; ++k) lg[k] = R(0);
-        } else if (x == a.nx - 2) {
+        }
+        if (a.fuse_neumann) {
 #pragma unroll
-            for (int k = 0; k < 7; ++k) lg[k] += A.lg1[(uint32_t)k * ns + c + 1];
+            for (int k = 0; k < 7; ++k) {
+                const R right = __shfl_down_sync(0xffffffffu, lg[k], 1);
+                if (xhi) lg[k] = R(0);
+                else if (w & kXHi1) lg[k] += right;
+            }
         }
     }
-    R lphi = A.lphi1[c] + (x == a.nx - 1 ? A.wl : R(0));
+    R lphi = A.lphi1[c] + (xhi ? A.wl : R(0));
     R lS = R(0), lux = R(0), luy = R(0), luz = R(0);
     R bsum = lphi;
 #pragma unroll
@@ -184,9 +309,11 @@ __global__ void __launch_bounds__(256, kAdjBlocks<T>) k_adj_cell(const AdjArgs<T
         else if (k == 5) luz += t;
         else if (k == 6) luz -= t;
     }
-    R lgo[7];
+    if (active) {
 #pragma unroll
-    for (int k = 0; k < 7; ++k) lgo[k] = (R(1) - om) * lg[k] + (phi_free ? bsum : R(0));
+        for (int k = 0; k < 7; ++k)
+            A.lgi[(uint32_t)k * ns + c] = (R(1) - om) * lg[k] + (phi_free ? bsum : R(0));
+    }
 
     // ---- adjoint of the LDF source ----
     R lq = A.lq1[c];
@@ -219,11 +346,70 @@ __global__ void __launch_bounds__(256, kAdjBlocks<T>) k_adj_cell(const AdjArgs<T
         lq = lq - a.iso_k * ldq;
         lphi0 = cfree ? lqeq * dqeq_dce : R(0);
     }
+    if (active) {
+        A.lphi0[c] = lphi0;
+        A.lq0[c] = lq;
+    }
 
     // ---- adjoint of the NS part ----
-    R lf[19];
+    pdl_launch_dependents();
+    // The NEQ inlet in the fused representation: the stored x = 0 populations of
+    // X_{s+1} are NEQ(f_{s+1} at x = 1) (src/boundary/ns/VelocityDirichletNEQ.cu:49-96),
+    // f_B = feq(rho_N, u_BC) + f_N - feq(rho_N, u_N).  Per row, lane k (direction
+    // k) moves the x = 0 adjoint into the x = 1 cell through the transposed
+    // Jacobian (identity, the rho_N derivative of the two equilibria, the u_N
+    // derivative of feq(rho_N, u_N)); the x = 0 adjoint is cleared.  nx is even,
+    // so both cells are lanes of this warp.
+    if (a.fuse_inlet) {
+        R* const ln = line[threadIdx.x >> 5];
+        const bool on = lane < 19;
+        const int k = on ? lane : 0;
+        const R cx = (R)((int)((kPX >> k) & 1u) - (int)((kMX >> k) & 1u));
+        const R cy = (R)((int)((kPY >> k) & 1u) - (int)((kMY >> k) & 1u));
+        const R cz = (R)((int)((kPZ >> k) & 1u) - (int)((kMZ >> k) & 1u));
+        const R wk = k == 0 ? R(1) / R(3) : (k < 7 ? R(1) / R(18) : R(1) / R(36));
+        for (uint32_t m = __ballot_sync(0xffffffffu, active && (w & kXLo1)); m; m &= m - 1u) {
+            const int src = __ffs(m) - 1;
+            const uint32_t c1 = cg - (uint32_t)lane + (uint32_t)src;   // the x = 1 cell
+            R* const side = A.x1 + ((uint32_t)k * a.rows_stride + fastdiv(c1, a.div_nx));
+            const R fN = on ? *side : R(0);
+            if (on) *side = Pop<T>::ld(a.fA + (uint32_t)k * ns + c1, fshift<T>(k, a.f_shift));
+            if (A.first) continue;
+            if (lane == src - 1) {
 #pragma unroll
-    for (int k = 0; k < 19; ++k) lf[k] = A.lf1[(uint32_t)k * ns + c];
+                for (int j = 0; j < 19; ++j) ln[j] = lf[j];
+            }
+            __syncwarp();
+            const R lB = on ? ln[k] : R(0);
+            const R r = warp_sum_r(fN);
+            const R jx = warp_sum_r(cx * fN), jy = warp_sum_r(cy * fN), jz = warp_sum_r(cz * fN);
+            const R inv = (r > R(0)) ? (R(1) / r) : R(0);
+            const R unx = jx * inv, uny = jy * inv, unz = jz * inv;
+            const R cuB = R(3) * (cx * a.uin_x + cy * a.uin_y + cz * a.uin_z);
+            const R cuN = R(3) * (cx * unx + cy * uny + cz * unz);
+            const R pB = R(1) + cuB + R(0.5) * cuB * cuB -
+                         R(1.5) * (a.uin_x * a.uin_x + a.uin_y * a.uin_y + a.uin_z * a.uin_z);
+            const R pN = R(1) + cuN + R(0.5) * cuN * cuN - R(1.5) * (unx * unx + uny * uny + unz * unz);
+            // d feq_k(r, u_N) / d u_N = w r (3 c + 9 (c.u) c - 3 u)
+            const R e = cx * unx + cy * uny + cz * unz;
+            const R gx = wk * r * (R(3) * cx + R(9) * e * cx - R(3) * unx);
+            const R gy = wk * r * (R(3) * cy + R(9) * e * cy - R(3) * uny);
+            const R gz = wk * r * (R(3) * cz + R(9) * e * cz - R(3) * unz);
+            const R s1 = warp_sum_r(lB * wk * (pB - pN));
+            const R Vx = warp_sum_r(lB * gx), Vy = warp_sum_r(lB * gy), Vz = warp_sum_r(lB * gz);
+            if (on) ln[k] = lB + s1 - ((cx - unx) * Vx + (cy - uny) * Vy + (cz - unz) * Vz) * inv;
+            __syncwarp();
+            if (lane == src) {
+#pragma unroll
+                for (int j = 0; j < 19; ++j) lf[j] += ln[j];
+            }
+            if (lane == src - 1) {
+#pragma unroll
+                for (int j = 0; j < 19; ++j) lf[j] = R(0);
+            }
+            __syncwarp();
+        }
+    }
     if (a.coupling && rp > R(0)) {
         // u_adv = j(fp) / rho(fp)
 #pragma unroll
@@ -231,21 +417,20 @@ __global__ void __launch_bounds__(256, kAdjBlocks<T>) k_adj_cell(const AdjArgs<T
             lf[k] += (((R)cx19(k) - uax) * lux + ((R)cy19(k) - uay) * luy + ((R)cz19(k) - uaz) * luz) * ip;
     }
     // pressure outlet: fp(nx-1) = feq_out(rho_out, u of fh(nx-2))
-    R lNx = R(0), lNy = R(0), lNz = R(0);
-    if (outlet) {
-#pragma unroll
-        for (int k = 0; k < 19; ++k) {
-            R gx, gy, gz;
-            dfeq_du(k, w19<R>(k), a.rho_out, uNx, uNy, uNz, gx, gy, gz);
-            lNx += lf[k] * gx; lNy += lf[k] * gy; lNz += lf[k] * gz;
-            lf[k] = R(0);
-        }
-    }
-    if (a.fuse_outlet) {
+    if (__any_sync(0xffffffffu, outlet)) {
+        R lNx = R(0), lNy = R(0), lNz = R(0);
+        if (outlet)
+            each19([&](auto k) {
+                constexpr int K = decltype(k)::value;
+                R gx, gy, gz;
+                dfeq_du<K>(a.rho_out, uNx, uNy, uNz, gx, gy, gz);
+                lNx += lf[K] * gx; lNy += lf[K] * gy; lNz += lf[K] * gz;
+                lf[K] = R(0);
+            }, Seq19{});
         const R rx = __shfl_down_sync(0xffffffffu, lNx, 1);
         const R ry = __shfl_down_sync(0xffffffffu, lNy, 1);
         const R rz = __shfl_down_sync(0xffffffffu, lNz, 1);
-        if (x == a.nx - 2 && rh > R(0)) {
+        if ((w & kXHi1) && rh > R(0)) {
 #pragma unroll
             for (int k = 0; k < 19; ++k)
                 lf[k] += (((R)cx19(k) - uhx) * rx + ((R)cy19(k) - uhy) * ry + ((R)cz19(k) - uhz) * rz) * ih;
@@ -254,13 +439,13 @@ __global__ void __launch_bounds__(256, kAdjBlocks<T>) k_adj_cell(const AdjArgs<T
     // collision: fh = fi + omega (feq(rho, u) - fi), u = por * j / rho
     if (!solid) {
         R As = R(0), Vx = R(0), Vy = R(0), Vz = R(0);
-#pragma unroll
-        for (int k = 0; k < 19; ++k) {
-            As += lf[k] * w19<R>(k) * poly19(k, ux, uy, uz);
+        each19([&](auto k) {
+            constexpr int K = decltype(k)::value;
+            As += lf[K] * w19<R>(K) * poly19<K>(ux, uy, uz, m15);
             R gx, gy, gz;
-            dfeq_du(k, w19<R>(k), rho, ux, uy, uz, gx, gy, gz);
-            Vx += lf[k] * gx; Vy += lf[k] * gy; Vz += lf[k] * gz;
-        }
+            dfeq_du<K>(rho, ux, uy, uz, gx, gy, gz);
+            Vx += lf[K] * gx; Vy += lf[K] * gy; Vz += lf[K] * gz;
+        }, Seq19{});
         const R sc = a.omega * por / rho;
 #pragma unroll
         for (int k = 0; k < 19; ++k)
@@ -272,126 +457,40 @@ __global__ void __launch_bounds__(256, kAdjBlocks<T>) k_adj_cell(const AdjArgs<T
     if (active) {
 #pragma unroll
         for (int k = 0; k < 19; ++k) A.lfi[(uint32_t)k * ns + c] = lf[k];
-#pragma unroll
-        for (int k = 0; k < 7; ++k) A.lgi[(uint32_t)k * ns + c] = lgo[k];
-        A.lphi0[c] = lphi0;
-        A.lq0[c] = lq;
     }
-    if (!active) { g0 = g1 = g2 = 0.0; }
-    double v[3] = {g0, g1, g2};
-    block_accumulate<3>(v, A.gpar);
-}
-
-// Transposed pull: lambda of every stored population of X_s from the
-// adjoints of the pulled values, then the NEQ inlet (x = 0 values derived
-// from x = 1 in the fused representation).
-template <typename T, typename QT, bool POROUS>
-__global__ void __launch_bounds__(256) k_adj_stream(const AdjArgs<T, QT> A, typename Pop<T>::R* __restrict__ lf0,
-                                                    typename Pop<T>::R* __restrict__ lg0)
-{
-    using R = typename Pop<T>::R;
-    const StepArgs<T, QT>& a = A.a;
-    const uint32_t cg = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = cg < (uint32_t)a.n;
-    const uint32_t c = active ? cg : (uint32_t)a.n - 1u;
-    int x, y, z;
-    cell_xyz(c, a.nx, a.ny, a.div_nx, a.div_nxy, x, y, z);
-    const Nbr nb(x, y, z, a.nx, a.ny, a.nz, a.px, a.py, a.pz);
-    const uint32_t w = __ldg(a.cellw + c);
-    const bool solid = !POROUS && (w & kSolid);
-    const uint32_t ns = a.ns;
-#pragma unroll
-    for (int j = 0; j < 19; ++j) {
-        const int o = opp19(j);
-        const int ox = cx19(o), oy = cy19(o), oz = cz19(o);
-        // the cell d = c + c_j pulls direction j from c (its direction-j source)
-        const bool in_o = nb.xo[1 - ox] && nb.yo[1 - oy] && nb.zo[1 - oz];
-        const uint32_t d = (uint32_t)(nb.xs[1 - ox] + nb.yr[1 - oy] + nb.zp[1 - oz]);
-        const bool link_o = !POROUS && ((w >> o) & 1u);
-        const int jx = cx19(j), jy = cy19(j), jz = cz19(j);
-        const bool in_j = nb.xo[1 - jx] && nb.yo[1 - jy] && nb.zo[1 - jz];
-        R v = R(0);
-        if (j == 0) {
-            v = A.lfi[c];
-        } else {
-            if (in_o && !link_o && !solid) v += A.lfi[(uint32_t)j * ns + d];
-            if (!in_j && !solid) v += A.lfi[(uint32_t)j * ns + c];
-            if (solid || (in_o && link_o)) v += A.lfi[(uint32_t)o * ns + c];
+    // this warp's share of the isotherm gradients, in a place of its own (summed by
+    // k_adj_fold at the end): no barrier and no atomics to three shared addresses
+    if (__any_sync(0xffffffffu, region && active)) {
+        const double s0 = warp_sum(active ? g0 : 0.0), s1 = warp_sum(active ? g1 : 0.0), s2 = warp_sum(active ? g2 : 0.0);
+        if (lane == 0) {
+            double* const p = A.gpar + (size_t)3 * (cg >> 5);
+            p[0] += s0; p[1] += s1; p[2] += s2;
         }
-        if (active) lf0[(uint32_t)j * ns + c] = v;
     }
-    R lg[7];
+}
+
+// the warps' shares of the isotherm gradients summed, in a fixed order
+__global__ void __launch_bounds__(1024) k_adj_fold(const double* __restrict__ part, int nwarps, double* __restrict__ out)
+{
+    __shared__ double sh[32][3];
+    double v[3] = {0.0, 0.0, 0.0};
+    for (int i = threadIdx.x; i < nwarps; i += blockDim.x)
 #pragma unroll
-    for (int j = 0; j < 7; ++j) {
-        const int jx = cx7(j), jy = cy7(j), jz = cz7(j);
-        const bool in_o = nb.xo[1 + jx] && nb.yo[1 + jy] && nb.zo[1 + jz];
-        const uint32_t d = (uint32_t)(nb.xs[1 + jx] + nb.yr[1 + jy] + nb.zp[1 + jz]);
-        const bool in_j = nb.xo[1 - jx] && nb.yo[1 - jy] && nb.zo[1 - jz];
-        R v = R(0);
-        if (j == 0) v = A.lgi[c];
-        else {
-            if (in_o) v += A.lgi[(uint32_t)j * ns + d];
-            if (!in_j) v += A.lgi[(uint32_t)j * ns + c];
+        for (int j = 0; j < 3; ++j) v[j] += part[(size_t)3 * i + j];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        v[j] = warp_sum(v[j]);
+        if (lane == 0) sh[wid][j] = v[j];
+    }
+    __syncthreads();
+    if (wid == 0) {
+        const int nw = blockDim.x >> 5;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const double s = warp_sum(lane < nw ? sh[lane][j] : 0.0);
+            if (lane == 0) out[j] = s;
         }
-        lg[j] = v;
-    }
-    if (active) {
-#pragma unroll
-        for (int k = 0; k < 7; ++k) lg0[(uint32_t)k * ns + c] = lg[k];
-    }
-}
-
-// The NEQ inlet in the fused representation: the stored x = 0 populations of
-// X_s are NEQ(f_s at x = 1) (src/boundary/ns/VelocityDirichletNEQ.cu:49-96),
-// f_B = feq(rho_N, u_BC) + f_N - feq(rho_N, u_N).  After the gather, one warp
-// per inlet row (lane k = direction k) moves the x = 0 adjoint into the x = 1
-// cell through the transposed Jacobian (identity, the rho_N derivative of the
-// two equilibria, the u_N derivative of feq(rho_N, u_N)) and clears x = 0.
-template <typename R>
-__device__ __forceinline__ R warp_sum_r(R v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-template <typename T, typename QT>
-__global__ void __launch_bounds__(256) k_adj_inlet(const AdjArgs<T, QT> A, typename Pop<T>::R* __restrict__ lf0)
-{
-    using R = typename Pop<T>::R;
-    const StepArgs<T, QT>& a = A.a;
-    const int row = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);   // warp-uniform
-    if (row >= a.ny * a.nz) return;
-    const int lane = threadIdx.x & 31;
-    const bool on = lane < 19;
-    const int k = on ? lane : 0;
-    const uint32_t ns = a.ns;
-    const uint32_t c0 = (uint32_t)row * (uint32_t)a.nx, c1 = c0 + 1u;
-    const R cx = (R)((int)((kPX >> k) & 1u) - (int)((kMX >> k) & 1u));
-    const R cy = (R)((int)((kPY >> k) & 1u) - (int)((kMY >> k) & 1u));
-    const R cz = (R)((int)((kPZ >> k) & 1u) - (int)((kMZ >> k) & 1u));
-    const R wk = k == 0 ? R(1) / R(3) : (k < 7 ? R(1) / R(18) : R(1) / R(36));
-    const R fN = on ? Pop<T>::ld(a.fA + (uint32_t)k * ns + c1, fshift<T>(k, a.f_shift)) : R(0);
-    const R lB = on ? lf0[(uint32_t)k * ns + c0] : R(0);
-    const R r = warp_sum_r(fN);
-    const R jx = warp_sum_r(cx * fN), jy = warp_sum_r(cy * fN), jz = warp_sum_r(cz * fN);
-    const R inv = (r > R(0)) ? (R(1) / r) : R(0);
-    const R unx = jx * inv, uny = jy * inv, unz = jz * inv;
-    const R cuB = R(3) * (cx * a.uin_x + cy * a.uin_y + cz * a.uin_z);
-    const R cuN = R(3) * (cx * unx + cy * uny + cz * unz);
-    const R pB = R(1) + cuB + R(0.5) * cuB * cuB - R(1.5) * (a.uin_x * a.uin_x + a.uin_y * a.uin_y + a.uin_z * a.uin_z);
-    const R pN = R(1) + cuN + R(0.5) * cuN * cuN - R(1.5) * (unx * unx + uny * uny + unz * unz);
-    // d feq_k(r, u_N) / d u_N = w r (3 c + 9 (c.u) c - 3 u)
-    const R e = cx * unx + cy * uny + cz * unz;
-    const R gx = wk * r * (R(3) * cx + R(9) * e * cx - R(3) * unx);
-    const R gy = wk * r * (R(3) * cy + R(9) * e * cy - R(3) * uny);
-    const R gz = wk * r * (R(3) * cz + R(9) * e * cz - R(3) * unz);
-    const R s1 = warp_sum_r(lB * wk * (pB - pN));
-    const R Vx = warp_sum_r(lB * gx), Vy = warp_sum_r(lB * gy), Vz = warp_sum_r(lB * gz);
-    if (on) {
-        R* p1 = lf0 + (uint32_t)k * ns + c1;
-        *p1 += lB + s1 - ((cx - unx) * Vx + (cy - uny) * Vy + (cz - unz) * Vz) * inv;
-        lf0[(uint32_t)k * ns + c0] = R(0);
     }
 }
 

@@ -299,8 +299,10 @@ struct StepArgs {
     T* __restrict__ fB;
     const T* __restrict__ gA;
     T* __restrict__ gB;
-    R* __restrict__ phi;
-    QT* __restrict__ q;
+    const R* phi;                         // C(s-1) and q before the step ...
+    const QT* q;
+    R* phi_out;                           // ... and after it (the same arrays, but for recomputed states)
+    QT* q_out;
     const uint32_t* __restrict__ cellw;   // per-cell flag word
     const R* __restrict__ porosity;       // porous collision
     const R* __restrict__ tau_ad;         // null: omega_ad for all cells
@@ -713,7 +715,7 @@ __device__ __forceinline__ void pull7_fast_all(typename Pop<T>::R* gi, const T* 
 
 // LDF source of a cell (src/reaction/LinearLDF.cu:13-48, src/reaction/LangmuirLDF.cu:7-41)
 // from its C(s-1) `cphi` and loading `qi`: S = -dq with dq = k (q_eq(C) - q);
-// `commit` stores q + dq to a.q[c]; `qn` receives the cell's loading after
+// `commit` stores q + dq to a.q_out[c]; `qn` receives the cell's loading after
 // the call.  Cells outside the region (or no isotherm) have S = 0.
 template <typename T, typename QT>
 __device__ __forceinline__ typename Pop<T>::R ldf_source_of(const StepArgs<T, QT>& a, uint32_t c, uint32_t w, bool commit,
@@ -736,7 +738,7 @@ __device__ __forceinline__ typename Pop<T>::R ldf_source_of(const StepArgs<T, QT
         const QT dq = (QT)a.iso_k * (qeq - qi);
         if (commit) {
             qn = qi + dq;
-            a.q[c] = qn;
+            a.q_out[c] = qn;
         }
         S = (R)(-dq);
     }
@@ -1119,10 +1121,10 @@ __device__ __forceinline__ void coupled_cell_dev(const StepArgs<T, QT>& a, uint3
     }
     if (do_ad) {
         store7(a, c, gn);
-        a.phi[c] = ph;
+        a.phi_out[c] = ph;
     }
     if (MON && active) {
-        mon->add((double)mrho, (double)ph, (double)a.q[c], (w & kXHi) ? (double)ph * (double)mux : 0.0,
+        mon->add((double)mrho, (double)ph, (double)a.q_out[c], (w & kXHi) ? (double)ph * (double)mux : 0.0,
                  !(mrho > 0.0f) || !isfinite(mrho) || !isfinite(ph));
     }
     if (a.fuse_inlet && xedge) fused_inlet(a, c, c, x, active);
@@ -1240,10 +1242,10 @@ __device__ __forceinline__ void coupled_cell(const StepArgs<T, QT>& a, uint32_t 
     }
     if (do_ad) {
         store7(a, c, gn);
-        a.phi[c] = ph;
+        a.phi_out[c] = ph;
     }
     if (MON && active) {
-        mon->add((double)mrho, (double)ph, (double)a.q[c], (w & kXHi) ? (double)ph * (double)mux : 0.0,
+        mon->add((double)mrho, (double)ph, (double)a.q_out[c], (w & kXHi) ? (double)ph * (double)mux : 0.0,
                  !(mrho > R(0)) || !isfinite(mrho) || !isfinite(ph));
     }
     if (a.fuse_inlet && xedge) fused_inlet(a, c, c, x, active);
@@ -1498,7 +1500,7 @@ __device__ __forceinline__ void coupled_cell_direct(const StepArgs<T, QT>& a, ui
         if (!(a.fuse_neumann && (w & kXHi) && (threadIdx.x & 31) == 0)) store7(a, c, gn, draw);
         // C is read back by the next step's LDF source, in the region only (not
         // writing the rest: FP32 512x256x128 581 -> 578 us a step)
-        if ((a.outputs & kOutC) || (w & kKeepC)) a.phi[c] = ph;
+        if ((a.outputs & kOutC) || (w & kKeepC)) a.phi_out[c] = ph;
     }
     if (xedge && (near0 | nearn)) direct_planes(a, near0, nearn, cg - (threadIdx.x & 31), st);
 }
@@ -1742,7 +1744,7 @@ __global__ void __launch_bounds__(256) k_ad_deferred(const StepArgs<T, QT> a, co
     pull7(a, c, nb, gi);
     const R ph = ad_collide(a, c, w, gi, ux, uy, uz, true, gn);
     store7(a, c, gn);
-    a.phi[c] = ph;
+    a.phi_out[c] = ph;
 }
 
 // Per-cell flag word from the bit-packed obstacle / region / deferred masks.

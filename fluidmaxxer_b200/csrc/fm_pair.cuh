@@ -499,13 +499,13 @@ __device__ __forceinline__ void pair_update(const StepArgs<T, QT>& a, uint32_t W
         if (active) gB[(uint32_t)k * ns2 + W] = PairG<T>::st(gn, k, a.g_shift, clo, chi);
     }
     if (active) {
-        a.phi[clo] = ph.x;
-        a.phi[chi] = ph.y;
+        a.phi_out[clo] = ph.x;
+        a.phi_out[chi] = ph.y;
     }
     if (MON && active) {
-        mon->add((double)mrho.x, (double)ph.x, (double)a.q[clo], 0.0,
+        mon->add((double)mrho.x, (double)ph.x, (double)a.q_out[clo], 0.0,
                  !(mrho.x > 0.0f) || !isfinite(mrho.x) || !isfinite(ph.x));
-        mon->add((double)mrho.y, (double)ph.y, (double)a.q[chi], (whi & kXHi) ? (double)ph.y * (double)mux : 0.0,
+        mon->add((double)mrho.y, (double)ph.y, (double)a.q_out[chi], (whi & kXHi) ? (double)ph.y * (double)mux : 0.0,
                  !(mrho.y > 0.0f) || !isfinite(mrho.y) || !isfinite(ph.y));
     }
     // the NEQ inlet of the next step on the low halves: x = 0 is the low half
