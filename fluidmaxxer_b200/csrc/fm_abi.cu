@@ -83,6 +83,11 @@ constexpr int kPrefetchWavePct = 54;
 // the same for the direct-planes step, which fetches only the flag words: 27%
 // (200 blocks), the middle of a flat range of 100-300
 constexpr int kHeadsWavePct = 27;
+// fm_get_fields: planes up to this size go to page-locked memory from the kernel.
+// One step and six FP32 fields, copies against kernel: 32x16x16 82 and 42 us,
+// 64x64x64 211 and 159, 128x128x64 (4 MiB planes) 594 and 544, 256x128x128 2093
+// and 2096; beyond, the copy engine's rate is the higher one.
+constexpr size_t kFieldsDirectBytes = (size_t)4 << 20;
 inline int grid_for(long long n, int block = kBlock) { return (int)((n + block - 1) / block); }
 
 enum BcKind { BC_NS_VEL_EQ, BC_NS_VEL_NEQ, BC_NS_PRESSURE, BC_NS_BOUNCEBACK, BC_AD_DIRICHLET, BC_AD_PULSE, BC_AD_NEUMANN };
@@ -172,6 +177,7 @@ struct fm_lattice {
     int staged_grid[4] = {0, 0, 0, 0};  // its resident blocks (persistent grid) per variant: BGK / porous x monitored
     size_t staged_smem[4] = {0, 0, 0, 0};   // ... and the shared memory they were sized for
     int* d_status = nullptr;            // device status word of the step kernels (fm_step_status)
+    bool status_used = false;           // a kernel that may set it has been launched
 };
 
 namespace {
@@ -701,6 +707,7 @@ int launch_staged(fm_lattice* L, fm::StepArgs<T, QT> a, bool mon, cudaStream_t s
     const uint32_t rows = (a.c_end - a.c_first) / (uint32_t)(L->p.nx / 2);
     const uint32_t tiles = (rows + a.st_rows - 1) / a.st_rows;
     *grid = (int)std::min<long long>(tiles, L->staged_grid[variant]);
+    L->status_used = true;
     kern<<<*grid, fm::kStageThreads, smem, st>>>(a);
     FM_CHECK_LAUNCH("k_pair_staged");
     *launched = true;
@@ -746,6 +753,15 @@ bool direct_planes(const fm::StepArgs<T, QT>& a)
     return a.fuse_outlet == a.fuse_neumann && a.nx >= fm::kDirectMinNx;
 }
 
+// The direct-planes step runs blocks of 128 threads up to kSmallCells cells, where
+// the last wave ends sooner: us a step with 128 and 256 threads, FP32 64x64x40 8.3
+// and 8.7, 128^3 76.0 and 76.8, 192x128x112 (2.8M) 97.9 and 96.6, 256x128x128 160
+// and 148; FP16 128^3 63.3 and 64.7, 436x124x206 390 and 339; FP64 128^3 137.7 and
+// 138.8, 436x124x206 704 and 699.  kResidentCells: what 148 SMs hold of the
+// 48-register forms at once.
+constexpr uint32_t kSmallCells = 2200000;
+constexpr uint32_t kResidentCells = 148 * 5 * 256;
+
 // `chained`: the previous work on `st` is a direct-planes step kernel of the
 // same run of steps, so this one may start while that one drains (programmatic
 // dependent launch; the kernel waits for it before its first pull).  Measured
@@ -760,16 +776,21 @@ void launch_coupled(const fm_lattice* L, int grid, cudaStream_t st, const fm::St
             if constexpr (fm::Pop<T>::kShifted) {
                 if (wide_offsets(L)) kern = fm::k_coupled_step<T, QT, POROUS, false, true, true>;
             }
+            const uint32_t cells = a.c_end - a.c_first;
+            const int block = cells <= kSmallCells ? kBlock / 2 : kBlock;
+            fm::StepArgs<T, QT> ad = a;
+            ad.pf_dist *= (uint32_t)(kBlock / block);
+            ad.early = cells > kResidentCells;
             cudaLaunchAttribute attr{};
             attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
             attr.val.programmaticStreamSerializationAllowed = 1;
             cudaLaunchConfig_t cfg{};
-            cfg.gridDim = dim3((unsigned)grid);
-            cfg.blockDim = dim3(kBlock);
+            cfg.gridDim = dim3((unsigned)grid_for(cells, block));
+            cfg.blockDim = dim3((unsigned)block);
             cfg.stream = st;
             cfg.attrs = &attr;
             cfg.numAttrs = chained ? 1 : 0;
-            cudaLaunchKernelEx(&cfg, kern, a);   // errors: the caller's FM_CHECK_LAUNCH
+            cudaLaunchKernelEx(&cfg, kern, ad);   // errors: the caller's FM_CHECK_LAUNCH
             return;
         }
     }
@@ -1018,15 +1039,31 @@ int init_state(fm_lattice* L)
     return FM_OK;
 }
 
+template <typename T>
+fm::FieldSource<T> field_source(const fm_lattice* L)
+{
+    return {(const T*)L->f[L->cur], L->ns, L->n, L->p.nx, (typename fm::Pop<T>::R)L->f_shift, pair_h(L), div_nx(L),
+            L->inlet_state == 1 ? (const T*)L->x0post : nullptr, L->rows_stride};
+}
+
 template <typename T, typename QT>
 int macros_to_tmp(fm_lattice* L)
 {
     using R = typename fm::Pop<T>::R;
     R* t = (R*)L->d_tmp;
-    fm::k_macros<T><<<grid_for(L->n), kBlock, 0, L->stream>>>((const T*)L->f[L->cur], L->ns, L->n, (R)L->f_shift, t,
-                                                             t + L->ns, t + 2 * L->ns, t + 3 * L->ns, pair_h(L),
-                                                             div_nx(L));
+    fm::k_macros<T><<<grid_for(L->n), kBlock, 0, L->stream>>>(field_source<T>(L), t, t + L->ns, t + 2 * L->ns,
+                                                             t + 3 * L->ns);
     FM_CHECK_LAUNCH("k_macros");
+    return FM_OK;
+}
+
+template <typename T, typename QT, typename OutT>
+int fields_direct(fm_lattice* L, const fm::FieldOuts<OutT>& o)
+{
+    using R = typename fm::Pop<T>::R;
+    fm::k_fields<T, QT, OutT><<<grid_for(L->n), kBlock, 0, L->stream>>>(field_source<T>(L), (const R*)L->phi,
+                                                                        (const QT*)L->q, o);
+    FM_CHECK_LAUNCH("k_fields");
     return FM_OK;
 }
 
@@ -1199,6 +1236,10 @@ int ensure_plain(fm_lattice* L)
 }
 template <typename T, typename QT> struct InitOp { static int run(fm_lattice* L) { return init_state<T, QT>(L); } };
 template <typename T, typename QT> struct MacroOp { static int run(fm_lattice* L) { return macros_to_tmp<T, QT>(L); } };
+template <typename T, typename QT> struct FieldsOp {
+    static int run(fm_lattice* L, const fm::FieldOuts<float>& o) { return fields_direct<T, QT, float>(L, o); }
+    static int run(fm_lattice* L, const fm::FieldOuts<double>& o) { return fields_direct<T, QT, double>(L, o); }
+};
 template <typename T, typename QT> struct SumOp { static int run(fm_lattice* L) { return domain_sums<T, QT>(L); } };
 template <typename T, typename QT> struct RangeSumOp {
     static int run(fm_lattice* L, int z0, int z1) { return range_sums<T, QT>(L, z0, z1); }
@@ -1708,6 +1749,7 @@ __global__ void k_widen(const float* __restrict__ src, double* __restrict__ dst,
 // fm_step_status (the word stays set until that call reads it)
 static int device_status(fm_lattice* L)
 {
+    if (!L->status_used) return FM_OK;
     int st = 0;
     FM_CUDA(cudaMemcpyAsync(&st, L->d_status, sizeof(int), cudaMemcpyDeviceToHost, L->stream));
     FM_CUDA(cudaStreamSynchronize(L->stream));
@@ -1769,6 +1811,21 @@ static int copy_real_plane_f32(fm_lattice* L, const void* src, float* out, size_
 // order and the copies run back to back.
 }  // extern "C"
 
+// The device address of page-locked host memory [p, p + bytes), or null.
+static void* mapped_host(const void* p, size_t bytes)
+{
+    cudaPointerAttributes lo{}, hi{};
+    const char* last = (const char*)p + bytes - 1;
+    if (cudaPointerGetAttributes(&lo, p) != cudaSuccess || cudaPointerGetAttributes(&hi, last) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    if (lo.type != cudaMemoryTypeHost || hi.type != cudaMemoryTypeHost || !lo.devicePointer || !hi.devicePointer ||
+        (char*)hi.devicePointer - (char*)lo.devicePointer != (ptrdiff_t)(bytes - 1))
+        return nullptr;
+    return lo.devicePointer;
+}
+
 template <typename OutT>
 static int get_fields_batched(fm_lattice* L, OutT* const out[6], size_t n)
 {
@@ -1776,8 +1833,23 @@ static int get_fields_batched(fm_lattice* L, OutT* const out[6], size_t n)
     if (!out || n != (size_t)L->n) return fail(FM_ERR_ARG, "fm_get_fields: size mismatch");
     const size_t N = (size_t)L->n;
     int rc = FM_OK;
+    // Small downloads are launches and copies, not bytes: one kernel writes the
+    // caller's buffers where they are page-locked.
+    if (N * sizeof(OutT) <= kFieldsDirectBytes) {
+        fm::FieldOuts<OutT> o{};
+        bool mapped = true;
+        for (int f = 0; f < 6 && mapped; ++f)
+            if (out[f]) {
+                o.p[f] = (OutT*)mapped_host(out[f], N * sizeof(OutT));
+                mapped = o.p[f] != nullptr;
+            }
+        if (mapped) {
+            if ((rc = dispatch<FieldsOp>(L, o))) return rc;
+            FM_CUDA(cudaStreamSynchronize(L->stream));
+            return device_status(L);
+        }
+    }
     if (out[0] || out[1] || out[2] || out[3]) {
-        if ((rc = ensure_plain(L))) return rc;
         if (!L->d_tmp && (rc = dev_alloc((char**)&L->d_tmp, (size_t)4 * L->ns * L->relt, L->stream))) return rc;
         if ((rc = dispatch<MacroOp>(L))) return rc;
     }
@@ -1814,8 +1886,6 @@ int fm_get_field_f32(fm_lattice* L, int field, float* out, size_t n)
     if (!out || n != (size_t)L->n) return fail(FM_ERR_ARG, "fm_get_field_f32: size mismatch");
     const size_t N = (size_t)L->n;
     if (field >= FM_FIELD_RHO && field <= FM_FIELD_UZ) {
-        int prc = ensure_plain(L);
-        if (prc) return prc;
         if (!L->d_tmp) {
             int rc = dev_alloc((char**)&L->d_tmp, (size_t)4 * L->ns * L->relt, L->stream);
             if (rc) return rc;
@@ -1838,8 +1908,6 @@ int fm_get_field(fm_lattice* L, int field, double* out, size_t n)
     if (!out || n != (size_t)L->n) return fail(FM_ERR_ARG, "fm_get_field: size mismatch");
     const size_t N = (size_t)L->n;
     if (field >= FM_FIELD_RHO && field <= FM_FIELD_UZ) {
-        int prc = ensure_plain(L);
-        if (prc) return prc;
         if (!L->d_tmp) {
             int rc = dev_alloc((char**)&L->d_tmp, (size_t)4 * L->ns * L->relt, L->stream);
             if (rc) return rc;
@@ -3299,6 +3367,7 @@ int fm_debug_layout(const fm_lattice* L, long long* plane_stride, int* precision
 int fm_debug_set_status(fm_lattice* L, int status)
 {
     if (check_lattice(L)) return FM_ERR_ARG;
+    L->status_used = true;
     FM_CUDA(cudaMemcpyAsync(L->d_status, &status, sizeof(int), cudaMemcpyHostToDevice, L->stream));
     FM_CUDA(cudaStreamSynchronize(L->stream));
     return FM_OK;

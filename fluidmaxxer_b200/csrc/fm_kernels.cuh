@@ -337,6 +337,7 @@ struct StepArgs {
     int* __restrict__ status;             // device status word: bit 0 a shared-memory stage wait gave up
     // direct planes only:
     int outputs;                          // what may be read before the next step: kOutX0 x0post, kOutC the C of every cell
+    int early;                            // the grid is more than one resident wave
     uint32_t rest;                        // kRest: both buffers hold resting obstacles' populations; 0: all are written
 };
 
@@ -1445,10 +1446,12 @@ __device__ __forceinline__ void coupled_cell_direct(const StepArgs<T, QT>& a, ui
             if (a.coupling || a.fuse_outlet) macro_velocity(fn, ux, uy, uz);
         }
     }
-    // the next step's grid may take its places: its blocks wait for this grid's end
-    // before their pulls.  Triggered here, not at the start: blocks placed beside
-    // running ones pile up on few SMs (64x32x32: 8.2 against 4.9 us a step)
-    pdl_launch_dependents();
+    // The next step's blocks may take their places; they wait for this grid's end
+    // before their pulls.  Not in a grid that is resident as a whole (its blocks'
+    // ends let the next grid in): blocks placed beside running ones pile up on few
+    // SMs (64x32x32: 8.2 us a step with the trigger at the start, 5.4 here, 4.9
+    // with none; 128x64x64: 20.7 here, 21.0 with none).
+    if (a.early) pdl_launch_dependents();
     bool st_own = active && moving;      // the lane stores its own cell's f
     uint32_t near0 = 0u, nearn = 0u;     // lanes at x = 1 (inlet) and x = nx-2 (outlet)
     if (xedge) {
@@ -1979,27 +1982,76 @@ __global__ void k_inlet_restore(T* __restrict__ f, long long ns, const int* __re
 // ---------------------------------------------------------------------------
 // macroscopic fields and FP64 reductions
 // ---------------------------------------------------------------------------
-// rho, u of the current f (src/core/Macros.cu:20-61) into planes of type R.
+// Where the populations of a lattice are read from for its fields: f in either
+// storage layout, and for the x = 0 cells the x0post side plane while f holds the
+// next step's inlet values there (null otherwise).
 template <typename T>
-__global__ void k_macros(const T* __restrict__ f, long long ns, int n, typename Pop<T>::R fsh,
-                         typename Pop<T>::R* __restrict__ rho, typename Pop<T>::R* __restrict__ ux,
-                         typename Pop<T>::R* __restrict__ uy, typename Pop<T>::R* __restrict__ uz, uint32_t pair_h,
-                         unsigned long long div_nx)
+struct FieldSource {
+    const T* __restrict__ f;
+    long long ns;
+    int n, nx;
+    typename Pop<T>::R fsh;
+    uint32_t pair_h;                      // pair_element
+    unsigned long long div_nx;
+    const T* __restrict__ x0post;
+    uint32_t rows_stride;
+};
+
+// rho, u of cell c (src/core/Macros.cu:20-61)
+template <typename T>
+__device__ __forceinline__ void cell_macros(const FieldSource<T>& s, int c, typename Pop<T>::R& r,
+                                            typename Pop<T>::R& ux, typename Pop<T>::R& uy, typename Pop<T>::R& uz)
+{
+    using R = typename Pop<T>::R;
+    const T* p = s.f + pair_element((uint32_t)c, s.pair_h, s.div_nx);
+    long long stride = s.ns;
+    if (s.x0post) {
+        const uint32_t row = fastdiv((uint32_t)c, s.div_nx);
+        if (row * (uint32_t)s.nx == (uint32_t)c) { p = s.x0post + row; stride = s.rows_stride; }
+    }
+    R v[19];
+#pragma unroll
+    for (int k = 0; k < 19; ++k) v[k] = Pop<T>::ld(p + k * stride, fshift<T>(k, s.fsh));
+    R jx, jy, jz;
+    moments19(v, r, jx, jy, jz, Seq19{});
+    const R inv = (r > R(0)) ? (R(1) / r) : R(0);
+    ux = jx * inv; uy = jy * inv; uz = jz * inv;
+}
+
+// rho, u into planes of type R
+template <typename T>
+__global__ void k_macros(const FieldSource<T> s, typename Pop<T>::R* __restrict__ rho,
+                         typename Pop<T>::R* __restrict__ ux, typename Pop<T>::R* __restrict__ uy,
+                         typename Pop<T>::R* __restrict__ uz)
+{
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= s.n) return;
+    cell_macros(s, c, rho[c], ux[c], uy[c], uz[c]);
+}
+
+// All six fields (null: skipped) in the output's type, written straight to
+// page-locked host memory: for lattices whose download is launches and copies
+// rather than bytes (fm_get_fields).
+template <typename OutT>
+struct FieldOuts {
+    OutT* p[6];
+};
+template <typename T, typename QT, typename OutT>
+__global__ void k_fields(const FieldSource<T> s, const typename Pop<T>::R* __restrict__ phi, const QT* __restrict__ q,
+                         const FieldOuts<OutT> o)
 {
     using R = typename Pop<T>::R;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n) return;
-    const uint32_t e = pair_element((uint32_t)c, pair_h, div_nx);
-    R v[19];
+    if (c >= s.n) return;
+    if (o.p[0] || o.p[1] || o.p[2] || o.p[3]) {
+        R v[4];
+        cell_macros(s, c, v[0], v[1], v[2], v[3]);
 #pragma unroll
-    for (int k = 0; k < 19; ++k) v[k] = Pop<T>::ld(f + (long long)k * ns + e, fshift<T>(k, fsh));
-    R r, jx, jy, jz;
-    moments19(v, r, jx, jy, jz, Seq19{});
-    const R inv = (r > R(0)) ? (R(1) / r) : R(0);
-    rho[c] = r;
-    ux[c] = jx * inv;
-    uy[c] = jy * inv;
-    uz[c] = jz * inv;
+        for (int j = 0; j < 4; ++j)
+            if (o.p[j]) o.p[j][c] = (OutT)v[j];
+    }
+    if (o.p[4]) o.p[4][c] = (OutT)phi[c];
+    if (o.p[5]) o.p[5][c] = (OutT)q[c];
 }
 
 // Block-reduce NV values per thread and add them to acc[0..NV) in FP64.
