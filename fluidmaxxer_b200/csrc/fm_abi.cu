@@ -780,7 +780,7 @@ void launch_coupled(const fm_lattice* L, int grid, cudaStream_t st, const fm::St
             const int block = cells <= kSmallCells ? kBlock / 2 : kBlock;
             fm::StepArgs<T, QT> ad = a;
             ad.pf_dist *= (uint32_t)(kBlock / block);
-            ad.early = cells > kResidentCells;
+            ad.early = L->elt >= 4 && cells > kResidentCells;
             cudaLaunchAttribute attr{};
             attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
             attr.val.programmaticStreamSerializationAllowed = 1;

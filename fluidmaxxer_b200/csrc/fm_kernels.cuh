@@ -115,45 +115,78 @@ __device__ __forceinline__ R cdot(R ux, R uy, R uz)
 // population storage: FP32 / FP64 as is; FP16 / BF16 hold the value minus a
 // shift (w_i rho0 for f, w_i c_shift for g) and compute in FP32.
 // ---------------------------------------------------------------------------
+// Loads of populations.  Ordinary coherent loads: a step launched while its
+// predecessor drains reads what that one wrote, which the read-only path does
+// not cover, and as volatile asm they stay behind pdl_wait.  The L2 fetch size
+// follows what the neighbours need: 256 B for 4- and 2-byte populations (FP16
+// 512x256x256 1035 against 1039 us a step at the default), 64 B for FP64, whose
+// resting obstacles leave gaps (2152 against 2217).
+__device__ __forceinline__ float ld_pop(const float* p)
+{
+    float v;
+    asm volatile("ld.global.L2::256B.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ double ld_pop(const double* p)
+{
+    double v;
+    asm volatile("ld.global.L2::64B.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ unsigned short ld_pop(const unsigned short* p)
+{
+    unsigned short v;
+    asm volatile("ld.global.L2::256B.u16 %0, [%1];" : "=h"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ __half ld_pop(const __half* p)
+{
+    return __ushort_as_half(ld_pop(reinterpret_cast<const unsigned short*>(p)));
+}
+__device__ __forceinline__ __nv_bfloat16 ld_pop(const __nv_bfloat16* p)
+{
+    return __ushort_as_bfloat16(ld_pop(reinterpret_cast<const unsigned short*>(p)));
+}
+
 template <typename T> struct Pop;
 template <> struct Pop<float> {
     using R = float;
     static constexpr bool kShifted = false;
-    __device__ static __forceinline__ R ld(const float* p, R) { return __ldg(p); }
+    __device__ static __forceinline__ R ld(const float* p, R) { return ld_pop(p); }
     __device__ static __forceinline__ R ld_coherent(const float* p, R) { return *p; }
     __device__ static __forceinline__ void st(float* p, R v, R) { *p = v; }
-    __device__ static __forceinline__ R ld_raw(const float* p) { return __ldg(p); }
+    __device__ static __forceinline__ R ld_raw(const float* p) { return ld_pop(p); }
     __device__ static __forceinline__ void st_raw(float* p, R v) { *p = v; }
 };
 template <> struct Pop<double> {
     using R = double;
     static constexpr bool kShifted = false;
-    __device__ static __forceinline__ R ld(const double* p, R) { return __ldg(p); }
+    __device__ static __forceinline__ R ld(const double* p, R) { return ld_pop(p); }
     __device__ static __forceinline__ R ld_coherent(const double* p, R) { return *p; }
     __device__ static __forceinline__ void st(double* p, R v, R) { *p = v; }
-    __device__ static __forceinline__ R ld_raw(const double* p) { return __ldg(p); }
+    __device__ static __forceinline__ R ld_raw(const double* p) { return ld_pop(p); }
     __device__ static __forceinline__ void st_raw(double* p, R v) { *p = v; }
 };
 template <> struct Pop<__half> {
     using R = float;
     static constexpr bool kShifted = true;
-    __device__ static __forceinline__ R ld(const __half* p, R sh) { return __half2float(__ldg(p)) + sh; }
+    __device__ static __forceinline__ R ld(const __half* p, R sh) { return __half2float(ld_pop(p)) + sh; }
     __device__ static __forceinline__ R ld_coherent(const __half* p, R sh) { return __half2float(*p) + sh; }
     __device__ static __forceinline__ void st(__half* p, R v, R sh) { *p = __float2half_rn(v - sh); }
     // the stored value itself (the deviation from the shift)
-    __device__ static __forceinline__ R ld_raw(const __half* p) { return __half2float(__ldg(p)); }
+    __device__ static __forceinline__ R ld_raw(const __half* p) { return __half2float(ld_pop(p)); }
     __device__ static __forceinline__ void st_raw(__half* p, R v) { *p = __float2half_rn(v); }
 };
 template <> struct Pop<__nv_bfloat16> {
     using R = float;
     static constexpr bool kShifted = true;
-    __device__ static __forceinline__ R ld(const __nv_bfloat16* p, R sh) { return __bfloat162float(__ldg(p)) + sh; }
+    __device__ static __forceinline__ R ld(const __nv_bfloat16* p, R sh) { return __bfloat162float(ld_pop(p)) + sh; }
     __device__ static __forceinline__ R ld_coherent(const __nv_bfloat16* p, R sh)
     {
         return __bfloat162float(*p) + sh;
     }
     __device__ static __forceinline__ void st(__nv_bfloat16* p, R v, R sh) { *p = __float2bfloat16_rn(v - sh); }
-    __device__ static __forceinline__ R ld_raw(const __nv_bfloat16* p) { return __bfloat162float(__ldg(p)); }
+    __device__ static __forceinline__ R ld_raw(const __nv_bfloat16* p) { return __bfloat162float(ld_pop(p)); }
     __device__ static __forceinline__ void st_raw(__nv_bfloat16* p, R v) { *p = __float2bfloat16_rn(v); }
 };
 
@@ -167,14 +200,14 @@ template <> struct Pop<hq> {
     static constexpr bool kShifted = true;
     __device__ static __forceinline__ R ld(const hq* p, R sh)
     {
-        return __half2float(__ushort_as_half(__ldg(&p->bits))) + sh;
+        return __half2float(__ushort_as_half(ld_pop(&p->bits))) + sh;
     }
     __device__ static __forceinline__ R ld_coherent(const hq* p, R sh)
     {
         return __half2float(__ushort_as_half(p->bits)) + sh;
     }
     __device__ static __forceinline__ void st(hq* p, R v, R sh) { p->bits = __half_as_ushort(__float2half_rn(v - sh)); }
-    __device__ static __forceinline__ R ld_raw(const hq* p) { return __half2float(__ushort_as_half(__ldg(&p->bits))); }
+    __device__ static __forceinline__ R ld_raw(const hq* p) { return __half2float(__ushort_as_half(ld_pop(&p->bits))); }
     __device__ static __forceinline__ void st_raw(hq* p, R v) { p->bits = __half_as_ushort(__float2half_rn(v)); }
 };
 
@@ -214,7 +247,7 @@ template <> struct PopG<hq> {
     using R = float;
     __device__ static __forceinline__ R ld(const hq* p, int k, R)
     {
-        return (R)((int)__ldg(&p->bits) - kGZero) * (w7<R>(k) * kGStep);
+        return (R)((int)ld_pop(&p->bits) - kGZero) * (w7<R>(k) * kGStep);
     }
     // Stochastic rounding: floor(t + r) with r in [0, 1) from a hash of the
     // value's bits, the cell and the direction, so E[stored] = t and changes
