@@ -1811,10 +1811,12 @@ static int copy_real_plane_f32(fm_lattice* L, const void* src, float* out, size_
 // order and the copies run back to back.
 }  // extern "C"
 
-// The device address of page-locked host memory [p, p + bytes), or null.
-static void* mapped_host(const void* p, size_t bytes)
+// The device address of page-locked host memory [p, p + bytes), or null (also for
+// memory a kernel could not store `align`-byte values to).
+static void* mapped_host(const void* p, size_t bytes, size_t align)
 {
     cudaPointerAttributes lo{}, hi{};
+    if ((uintptr_t)p % align) return nullptr;
     const char* last = (const char*)p + bytes - 1;
     if (cudaPointerGetAttributes(&lo, p) != cudaSuccess || cudaPointerGetAttributes(&hi, last) != cudaSuccess) {
         cudaGetLastError();
@@ -1840,8 +1842,11 @@ static int get_fields_batched(fm_lattice* L, OutT* const out[6], size_t n)
         bool mapped = true;
         for (int f = 0; f < 6 && mapped; ++f)
             if (out[f]) {
-                o.p[f] = (OutT*)mapped_host(out[f], N * sizeof(OutT));
+                o.p[f] = (OutT*)mapped_host(out[f], N * sizeof(OutT), sizeof(OutT));
                 mapped = o.p[f] != nullptr;
+                // overlapping buffers keep the copies' order: the last field stays
+                for (int j = 0; j < f; ++j)
+                    mapped = mapped && (!out[j] || out[j] + N <= out[f] || out[f] + N <= out[j]);
             }
         if (mapped) {
             if ((rc = dispatch<FieldsOp>(L, o))) return rc;

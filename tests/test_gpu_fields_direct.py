@@ -53,6 +53,19 @@ def test_part_pinned_buffers_take_the_copies():
     L.close()
 
 
+def test_overlapping_buffers_keep_the_last_field():
+    import ctypes as C
+
+    p = problems.channel_small(5, 48, 10, 9)
+    L = lattice.from_problem(p, "f32")
+    L.step(30)
+    one = pinned(L.n, np.float32)
+    ptrs = (C.c_void_p * 6)(*[one.ctypes.data] * 6)
+    assert L._lib.fm_get_fields_f32(L.h, ptrs, L.n) == 0
+    assert np.array_equal(one, L.field("q", dtype=np.float32))
+    L.close()
+
+
 def test_pair_layout_fields():
     p = problems.channel_small(5, 64, 16, 16)
     L, M = lattice.from_problem(p, "f16"), lattice.from_problem(p, "f16")
