@@ -348,8 +348,8 @@ int fm_bench_pull_copy(fm_lattice* lat, int reps, double* ms_per_rep, double* by
  * sum(rho) of the stored populations, sum(C), sum(q), the outlet flux
  * sum(C u_x) over the x = nx-1 cells, and the number of cells whose rho is not
  * positive or whose rho or C is not finite (a divergence status).  Needs
- * every boundary inside the fused step (fm_launches_per_step == 1), else
- * fm_step returns FM_ERR_UNSUPPORTED.  fm_get_monitor copies up to `capacity`
+ * every boundary inside the fused step (fm_launches_per_step == 1) and, with
+ * boundaries, even nx, else fm_step returns FM_ERR_UNSUPPORTED.  fm_get_monitor copies up to `capacity`
  * rows of 6 doubles (step, mass, C, q, outlet flux, bad cells) and writes the
  * number of rows; fm_init_equilibrium and fm_set_monitor restart the rows.
  * every = 0 turns the monitor off. */
@@ -444,8 +444,8 @@ int fm_unpack_zhalo(fm_lattice* lat, int z, int dir, const void* d_buf);
  * count, outlet sample).  Planes not stepped keep stale populations in the
  * buffer being written (ghost planes, whose crossing populations the halo
  * unpack then supplies).  Requires a lattice whose step is one launch
- * (fm_launches_per_step == 1) and nx*ny a multiple of 64; FM_ERR_UNSUPPORTED
- * otherwise.  fm_step and fm_reduce_zrange refuse while a step is open. */
+ * (fm_launches_per_step == 1) with, where it has boundaries, even nx, and nx*ny
+ * a multiple of 64; FM_ERR_UNSUPPORTED otherwise.  fm_step and fm_reduce_zrange refuse while a step is open. */
 int fm_step_planes(fm_lattice* lat, int z0, int z1);
 int fm_step_finish(fm_lattice* lat);
 /* Sums of rho, C and q over the z-planes [z0, z1) (the interior of a slab),
