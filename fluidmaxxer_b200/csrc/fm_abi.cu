@@ -152,6 +152,7 @@ struct fm_lattice {
     bool dirty = true;                  // flags / fusion need rebuilding
     bool split_open = false;            // a step begun by fm_step_planes, not yet finished
     bool rest = false;                  // both buffers hold every obstacle off the x-faces at the rest equilibrium
+    bool moved = false;                 // a step kernel has written f since fm_init_equilibrium (trials included)
     bool chain = false;                 // within fm_step: the last queued work is a step kernel the next one may chain to
     int fuse_outlet = 0, fuse_neumann = 0, fuse_dirichlet = 0;
     uint32_t pf_dist = 0;               // L2 prefetch distance of the fused kernel (blocks)
@@ -817,6 +818,7 @@ int launch_step(fm_lattice* L, bool last)
     const long long s = L->step + 1;
     const int A = L->cur, B = 1 - L->cur;
     cudaStream_t st = L->stream;
+    L->moved = true;
     const bool mon = L->mon_every > 0 && s % L->mon_every == 0;
     T* fA = (T*)L->f[A];
     T* fB = (T*)L->f[B];
@@ -939,6 +941,7 @@ int launch_planes(fm_lattice* L, int z0, int z1)
     fm::StepArgs<T, QT> a = make_args<T, QT>(L);
     const uint32_t nxy = (uint32_t)L->p.nx * (uint32_t)L->p.ny;
     cudaStream_t st = L->stream;
+    L->moved = true;
     if constexpr (fm::Pop<T>::kShifted) {
         if (L->layout == 1) {
             a.c_first = (uint32_t)z0 * (nxy / 2);
@@ -1272,7 +1275,9 @@ int ensure_layout(fm_lattice* L)
 }
 
 // Populations of f[cur] or f[1-cur], or the obstacles themselves, changed from
-// outside the step: obstacles may not be at rest any more.
+// outside the step: obstacles may not be at rest any more.  (Obstacles placed
+// before any step are: `moved`, not the step count, tells, since the trials of
+// fm_batch_autotune write both buffers and leave the count where it was.)
 void rest_unknown(fm_lattice* L)
 {
     if (L->rest) L->dirty = true;
@@ -1426,7 +1431,7 @@ int fm_set_obstacle_mask(fm_lattice* L, const uint8_t* mask, size_t n)
 {
     if (check_mask(L, mask, n, "NSLattice::setObstacleMask:")) return FM_ERR_ARG;
     std::vector<uint32_t> bits = pack_bits(mask, n, L->nwords);
-    if (L->step > 0 || L->split_open) rest_unknown(L);
+    if (L->moved) rest_unknown(L);
     FM_CUDA(cudaMemcpyAsync(L->solid, bits.data(), bits.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, L->stream));
     FM_CUDA(cudaStreamSynchronize(L->stream));
     L->dirty = true;
@@ -1441,7 +1446,7 @@ int fm_set_obstacle_bits(fm_lattice* L, const uint32_t* bits, size_t nwords)
     std::memcpy(b.data(), bits, nwords * sizeof(uint32_t));
     const size_t tail = (size_t)L->n & 31;   // clear bits past the last cell
     if (tail) b[(size_t)L->n >> 5] &= (1u << tail) - 1u;
-    if (L->step > 0 || L->split_open) rest_unknown(L);
+    if (L->moved) rest_unknown(L);
     FM_CUDA(cudaMemcpyAsync(L->solid, b.data(), b.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, L->stream));
     FM_CUDA(cudaStreamSynchronize(L->stream));
     L->dirty = true;
@@ -1697,6 +1702,7 @@ int fm_init_equilibrium(fm_lattice* L)
     const bool rest = L->collision == FM_COLL_BGK && L->p.rho0 > 1e-30 && L->p.rho0 < 1e30;
     if (rest != L->rest) L->dirty = true;
     L->rest = rest;
+    L->moved = false;
     L->initialised = true;
     if (L->nprobe && L->probe_every > 0) return take_sample(L);
     return FM_OK;
@@ -2513,6 +2519,7 @@ int batch_ready(fm_batch* B)
         if (!rc) rc = ensure_layout(L);
         if (!rc && L->fuse_inlet && L->inlet_state == 0) rc = dispatch<InletFusedOp>(L);
         if (rc) return rc;
+        L->moved = true;
         FM_CUDA(cudaEventRecord(B->ev, L->stream));
         FM_CUDA(cudaStreamWaitEvent(B->stream, B->ev, 0));
     }
