@@ -108,6 +108,7 @@ SIGNATURES = {
     "fm_launches_per_step": (_i, [_vp]),
     "fm_debug_layout": (_i, [_vp, C.POINTER(C.c_longlong), C.POINTER(_i)]),
     "fm_debug_set_status": (_i, [_vp, _i]),
+    "fm_debug_host_span": (_i, [_vp, _vp, _vp, _i, C.c_ulonglong, _sz, _sz]),
 }
 
 _LIB = None

@@ -10,6 +10,7 @@
 #include "fm_pair.cuh"
 #include "fm_adjoint.cuh"
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 #if defined(__SSE2__) && !defined(__CUDA_ARCH__)
 #include <emmintrin.h>
@@ -1821,21 +1822,71 @@ static int copy_real_plane_f32(fm_lattice* L, const void* src, float* out, size_
 // order and the copies run back to back.
 }  // extern "C"
 
-// The device address of page-locked host memory [p, p + bytes), or null (also for
-// memory a kernel could not store `align`-byte values to).
-static void* mapped_host(const void* p, size_t bytes, size_t align)
+// The page-locked allocation or registration a host address lies in.
+struct HostRange {
+    unsigned long long start = 0, size = 0;
+    bool writable = false;   // host memory the current device may store to, at the host's own address
+};
+
+// Whether page-locked ranges the device may store to cover [p, p + bytes) without
+// a gap, for values of `align` bytes; query(address, range&) tells the range an
+// address lies in.
+template <typename Query>
+static bool host_span_writable(unsigned long long p, size_t bytes, size_t align, Query query)
 {
-    cudaPointerAttributes lo{}, hi{};
-    if ((uintptr_t)p % align) return nullptr;
-    const char* last = (const char*)p + bytes - 1;
-    if (cudaPointerGetAttributes(&lo, p) != cudaSuccess || cudaPointerGetAttributes(&hi, last) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
+    if (p % align) return false;
+    for (unsigned long long at = p, end = p + bytes; at < end;) {
+        HostRange r;
+        if (!query(at, r) || !r.writable || r.start > at || r.size <= at - r.start) return false;
+        at = r.start + r.size;
     }
-    if (lo.type != cudaMemoryTypeHost || hi.type != cudaMemoryTypeHost || !lo.devicePointer || !hi.devicePointer ||
-        (char*)hi.devicePointer - (char*)lo.devicePointer != (ptrdiff_t)(bytes - 1))
-        return nullptr;
-    return lo.devicePointer;
+    return true;
+}
+
+// The range of `at` as the driver knows it (false where the driver entry point is
+// unavailable or the address is not CUDA's).  Memory registered read-only is not
+// writable, nor is managed memory page-locked.
+static bool driver_host_range(unsigned long long at, HostRange& r)
+{
+    using GetAttributes = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+    static GetAttributes fn = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &p, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            p = nullptr;
+        cudaGetLastError();
+        return reinterpret_cast<GetAttributes>(p);
+    }();
+    if (!fn) return false;
+    CUpointer_attribute what[6] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE,      CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                   CU_POINTER_ATTRIBUTE_DEVICE_POINTER,   CU_POINTER_ATTRIBUTE_ACCESS_FLAGS,
+                                   CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    unsigned long long v[6] = {};   // each value is 1, 4 or 8 bytes
+    void* out[6];
+    for (int i = 0; i < 6; ++i) out[i] = &v[i];
+    if (fn(6, what, out, (CUdeviceptr)at) != CUDA_SUCCESS) return false;
+    r.writable = v[0] == CU_MEMORYTYPE_HOST && !v[1] && v[2] == at && v[3] == CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE;
+    r.start = v[4];
+    r.size = v[5];
+    return true;
+}
+
+extern "C" int fm_debug_host_span(const unsigned long long* starts, const unsigned long long* sizes,
+                                  const int* writable, int count, unsigned long long p, size_t bytes, size_t align)
+{
+    if (count < 0 || (count && (!starts || !sizes || !writable)) || !align)
+        return fail(FM_ERR_ARG, "fm_debug_host_span: bad arguments");
+    return host_span_writable(p, bytes, align, [&](unsigned long long at, HostRange& r) {
+        for (int i = 0; i < count; ++i)
+            if (at >= starts[i] && at - starts[i] < sizes[i]) {
+                r.start = starts[i];
+                r.size = sizes[i];
+                r.writable = writable[i] != 0;
+                return true;
+            }
+        return false;
+    });
 }
 
 template <typename OutT>
@@ -1852,8 +1903,9 @@ static int get_fields_batched(fm_lattice* L, OutT* const out[6], size_t n)
         bool mapped = true;
         for (int f = 0; f < 6 && mapped; ++f)
             if (out[f]) {
-                o.p[f] = (OutT*)mapped_host(out[f], N * sizeof(OutT), sizeof(OutT));
-                mapped = o.p[f] != nullptr;
+                o.p[f] = out[f];
+                mapped = host_span_writable((unsigned long long)(uintptr_t)out[f], N * sizeof(OutT), sizeof(OutT),
+                                            driver_host_range);
                 // overlapping buffers keep the copies' order: the last field stays
                 for (int j = 0; j < f; ++j)
                     mapped = mapped && (!out[j] || out[j] + N <= out[f] || out[f] + N <= out[j]);

@@ -459,6 +459,12 @@ int fm_debug_layout(const fm_lattice* lat, long long* plane_stride, int* precisi
  * the host-side detection of a device wait that gave up can be tested without
  * making a kernel wait run out. */
 int fm_debug_set_status(fm_lattice* lat, int status);
+/* Test aid: 1 when page-locked ranges [starts[i], starts[i] + sizes[i]) with
+ * writable[i] set cover [p, p + bytes) without a gap and p is a multiple of
+ * `align`, else 0: the rule by which fm_get_fields lets a kernel store to the
+ * caller's buffer.  Host arithmetic on made-up addresses, nothing is read. */
+int fm_debug_host_span(const unsigned long long* starts, const unsigned long long* sizes, const int* writable,
+                       int count, unsigned long long p, size_t bytes, size_t align);
 
 #ifdef __cplusplus
 }
