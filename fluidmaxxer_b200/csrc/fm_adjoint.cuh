@@ -34,21 +34,54 @@
 
 namespace fm {
 
+// Ordinary coherent loads that stay behind pdl_wait (as ld_pop); with a condition,
+// predicated, and 0 where it is false.
+__device__ __forceinline__ float ld_adj(const float* p)
+{
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ double ld_adj(const double* p)
+{
+    double v;
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float ld_adj(const float* p, bool on)
+{
+    float v;
+    asm volatile("{ .reg .pred q; setp.ne.u32 q, %2, 0; mov.f32 %0, 0f00000000; @q ld.global.f32 %0, [%1]; }"
+                 : "=&f"(v) : "l"(p), "r"((uint32_t)on));
+    return v;
+}
+__device__ __forceinline__ double ld_adj(const double* p, bool on)
+{
+    double v;
+    asm volatile("{ .reg .pred q; setp.ne.u32 q, %2, 0; mov.f64 %0, 0d0000000000000000; @q ld.global.f64 %0, [%1]; }"
+                 : "=&d"(v) : "l"(p), "r"((uint32_t)on));
+    return v;
+}
+
 template <typename T, typename QT>
 struct AdjArgs {
     using R = typename Pop<T>::R;
     StepArgs<T, QT> a;              // forward step from X_s (fA = f_s, gA = g_s, phi = phi_s, q = q_s)
-    const R* __restrict__ lfi1;     // adjoints of the D3Q19 populations step s+2 pulled [19][ns]
-    const R* __restrict__ lgi1;     // the same of the D3Q7 populations [7][ns]
-    const R* __restrict__ lphi1;    // lambda phi_{s+1}
-    const R* __restrict__ lq1;      // lambda q_{s+1}
-    R* __restrict__ lfi;            // out: adjoints of the D3Q19 populations step s+1 pulls
-    R* __restrict__ lgi;            // out: the same of the D3Q7 populations
-    R* __restrict__ lphi0;          // out: lambda phi_s
-    R* __restrict__ lq0;            // out: lambda q_s
-    R* __restrict__ x1;             // [19][rows]: f_{s+1} at x = 1 in, f_s at x = 1 out
-    double* __restrict__ gpor;      // += dL/d porosity per cell (porous collision)
-    double* __restrict__ gpar;      // += dL/d (isotherm a, b, k), per warp [warps][3]
+    // The launches before a backward step write all of these, and it may start
+    // while they drain: inputs are read by ld_adj behind pdl_wait, and nothing is
+    // declared __restrict__, which would let a load take the read-only path or
+    // move above the wait.
+    const R* lfi1;                  // adjoints of the D3Q19 populations step s+2 pulled [19][ns]
+    const R* lgi1;                  // the same of the D3Q7 populations [7][ns]
+    const R* lphi1;                 // lambda phi_{s+1}
+    const R* lq1;                   // lambda q_{s+1}
+    R* lfi;                         // out: adjoints of the D3Q19 populations step s+1 pulls
+    R* lgi;                         // out: the same of the D3Q7 populations
+    R* lphi0;                       // out: lambda phi_s
+    R* lq0;                         // out: lambda q_s
+    R* x1;                          // [19][rows]: f_{s+1} at x = 1 in, f_s at x = 1 out
+    double* gpor;                   // += dL/d porosity per cell (porous collision)
+    double* gpar;                   // += dL/d (isotherm a, b, k), per warp [warps][3]
     R wl;                           // loss weight on phi_{s+1} of the outlet plane (0: not sampled)
     int first;                      // no backward step before: lfi1, lgi1 are zero
 };
@@ -100,39 +133,44 @@ __device__ __forceinline__ R warp_sum_r(R v)
 // its own opposite direction (a link to an obstacle at c + c_J, or an obstacle
 // cell, whose bits lk 1..18 are all set).
 template <int J, bool BB, typename R>
-__device__ __forceinline__ R gather19_fast(const R* __restrict__ base, uint32_t ns, int nx, int nxy, int px, bool xlo,
+__device__ __forceinline__ R gather19_fast(const R* base, uint32_t ns, int nx, int nxy, int px, bool xlo,
                                            bool xhi, uint32_t lk, bool solid)
 {
     constexpr int CX = cx19(J), CY = cy19(J), CZ = cz19(J), O = opp19(J);
-    if (J == 0) return base[0];
+    if (J == 0) return ld_adj(base);
     const bool own = BB && ((lk >> O) & 1u);
     const bool out = CX != 0 && (CX > 0 ? xhi : xlo);    // c + c_J beyond an x-face
     const bool keep = CX != 0 && (CX > 0 ? xlo : xhi);   // c - c_J beyond an x-face: the cell kept its own value
     uint32_t off = (uint32_t)J * ns + (uint32_t)(CX + CY * nx + CZ * nxy);
     if (out) off -= (uint32_t)(CX * nx);                 // periodic x
     if (own) off = (uint32_t)O * ns;
-    R v = (out && !px && !own) ? R(0) : base[off];
-    if (keep && !px && !solid) v += base[(uint32_t)J * ns];
+    R v = ld_adj(base + off);                            // in the array in any case
+    if (out && !px && !own) v = R(0);
+    if (CX != 0) {
+        const bool too = keep && !px && !solid;
+        const R k = ld_adj(base + (uint32_t)J * ns, too);
+        if (too) v += k;
+    }
     return v;
 }
 // the same for any cell
 template <int J, bool BB, typename R>
-__device__ __forceinline__ R gather19(const R* __restrict__ l, uint32_t ns, uint32_t c, const Nbr& nb, uint32_t w,
+__device__ __forceinline__ R gather19(const R* l, uint32_t ns, uint32_t c, const Nbr& nb, uint32_t w,
                                       bool solid)
 {
     constexpr int CX = cx19(J), CY = cy19(J), CZ = cz19(J), O = opp19(J);
-    if (J == 0) return l[c];
+    if (J == 0) return ld_adj(l + c);
     const bool in_o = nb.inside<-CX, -CY, -CZ>(), in_j = nb.inside<CX, CY, CZ>();
     const bool link = BB && ((w >> O) & 1u);
     R v = R(0);
-    if (in_o && !link && !solid) v += l[(uint32_t)J * ns + (uint32_t)nb.src<-CX, -CY, -CZ>()];
-    if (!in_j && !solid) v += l[(uint32_t)J * ns + c];
-    if (solid || (in_o && link)) v += l[(uint32_t)O * ns + c];
+    if (in_o && !link && !solid) v += ld_adj(l + ((uint32_t)J * ns + (uint32_t)nb.src<-CX, -CY, -CZ>()));
+    if (!in_j && !solid) v += ld_adj(l + ((uint32_t)J * ns + c));
+    if (solid || (in_o && link)) v += ld_adj(l + ((uint32_t)O * ns + c));
     return v;
 }
 // D3Q7 has no reflection
 template <int J, typename R>
-__device__ __forceinline__ R gather7_fast(const R* __restrict__ base, uint32_t ns, int nx, int nxy, int px, bool xlo,
+__device__ __forceinline__ R gather7_fast(const R* base, uint32_t ns, int nx, int nxy, int px, bool xlo,
                                           bool xhi)
 {
     return gather19_fast<J, false>(base, ns, nx, nxy, px, xlo, xhi, 0u, false);
@@ -286,7 +324,7 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjBlocks<T>) k_adj_step(const A
             }
         }
     }
-    R lphi = A.lphi1[c] + (xhi ? A.wl : R(0));
+    R lphi = ld_adj(A.lphi1 + c) + (xhi ? A.wl : R(0));
     R lS = R(0), lux = R(0), luy = R(0), luz = R(0);
     R bsum = lphi;
 #pragma unroll
@@ -316,14 +354,14 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjBlocks<T>) k_adj_step(const A
     }
 
     // ---- adjoint of the LDF source ----
-    R lq = A.lq1[c];
+    R lq = ld_adj(A.lq1 + c);
     R lphi0 = R(0);
     double g0 = 0.0, g1 = 0.0, g2 = 0.0;
     if (region) {
-        const R p0 = a.phi[c];
+        const R p0 = ld_adj(a.phi + c);
         const bool cfree = !(p0 < a.min_conc);
         const R ce = (cfree ? p0 : a.min_conc) - a.min_conc;
-        const R qi = (R)a.q[c];
+        const R qi = (R)ld_adj(a.q + c);
         R qeq, dqeq_dce, g_a, g_b;
         if (a.isotherm == 1) {
             qeq = a.iso_a * ce;
@@ -372,7 +410,7 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjBlocks<T>) k_adj_step(const A
             const int src = __ffs(m) - 1;
             const uint32_t c1 = cg - (uint32_t)lane + (uint32_t)src;   // the x = 1 cell
             R* const side = A.x1 + ((uint32_t)k * a.rows_stride + fastdiv(c1, a.div_nx));
-            const R fN = on ? *side : R(0);
+            const R fN = ld_adj(side, on);
             if (on) *side = Pop<T>::ld(a.fA + (uint32_t)k * ns + c1, fshift<T>(k, a.f_shift));
             if (A.first) continue;
             if (lane == src - 1) {
