@@ -20,6 +20,7 @@
 #include <unistd.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <condition_variable>
 #include <cstdio>
@@ -853,13 +854,6 @@ int launch_step(fm_lattice* L, bool last)
     a.outputs = (last ? fm::kOutX0 : 0) | (last || sampled ? fm::kOutC : 0);
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     if (L->profiling) {
-        if (L->prof_used + 2 > L->prof_ev.size()) {
-            for (int i = 0; i < 256; ++i) {
-                cudaEvent_t e;
-                FM_CUDA(cudaEventCreate(&e));
-                L->prof_ev.push_back(e);
-            }
-        }
         ev0 = L->prof_ev[L->prof_used];
         ev1 = L->prof_ev[L->prof_used + 1];
         L->prof_used += 2;
@@ -890,19 +884,8 @@ int launch_step(fm_lattice* L, bool last)
     }
     if (ev1) FM_CUDA(cudaEventRecord(ev1, st));
     if (mon) {
-        // the launch's partials folded into the next row of the monitor
+        // the launch's partials folded into the next row of the monitor (reserve_outputs)
         const int row = (int)L->mon_steps.size();
-        if (row >= L->mon_cap) {
-            const int cap = std::max(64, 2 * L->mon_cap);
-            double* nb = nullptr;
-            int rc = dev_alloc(&nb, (size_t)cap * fm::kMonN, st);
-            if (rc) return rc;
-            if (row)
-                FM_CUDA(cudaMemcpyAsync(nb, L->d_mon, sizeof(double) * fm::kMonN * row, cudaMemcpyDeviceToDevice, st));
-            dev_free(L->d_mon, st);
-            L->d_mon = nb;
-            L->mon_cap = cap;
-        }
         fm::k_monitor_fold<<<1, kBlock, 0, st>>>(L->d_mon_part, grid, L->d_mon + (size_t)row * fm::kMonN);
         FM_CHECK_LAUNCH("k_monitor_fold");
         L->mon_steps.push_back(s);
@@ -1004,6 +987,49 @@ int ensure_bt_capacity(fm_lattice* L, int need)
     L->d_bt = nb;
     L->bt_cap = cap;
     return FM_OK;
+}
+
+int ensure_mon_capacity(fm_lattice* L, int need)
+{
+    if (need <= L->mon_cap) return FM_OK;
+    const int rows = (int)L->mon_steps.size(), cap = std::max(need, std::max(64, 2 * L->mon_cap));
+    double* nb = nullptr;
+    int rc = dev_alloc(&nb, (size_t)cap * fm::kMonN, L->stream);
+    if (rc) return rc;
+    if (rows)
+        FM_CUDA(cudaMemcpyAsync(nb, L->d_mon, sizeof(double) * fm::kMonN * rows, cudaMemcpyDeviceToDevice, L->stream));
+    dev_free(L->d_mon, L->stream);
+    L->d_mon = nb;
+    L->mon_cap = cap;
+    return FM_OK;
+}
+
+// Everything the next `nsteps` steps need memory or events for: the samples of
+// the breakthrough series, the monitor's rows, the profiler's events.  Taken
+// before the first step, so a call that cannot have them fails with the lattice
+// untouched: between its first and last step C is up to date in the region only
+// and x0post not at all (StepArgs::outputs).
+int reserve_outputs(fm_lattice* L, int nsteps)
+{
+    const auto due = [&](int every) { return (L->step + nsteps) / every - L->step / every; };
+    int rc = FM_OK;
+    if (L->nprobe && L->probe_every > 0) {
+        const long long need = L->bt_count + due(L->probe_every);
+        if (need > INT_MAX) return fail(FM_ERR_NOMEM, "fm_step: more samples than a series holds");
+        rc = ensure_bt_capacity(L, (int)need);
+    }
+    if (!rc && L->mon_every > 0) {
+        const long long need = (long long)L->mon_steps.size() + due(L->mon_every);
+        if (need > INT_MAX) return fail(FM_ERR_NOMEM, "fm_step: more rows than the monitor holds");
+        rc = ensure_mon_capacity(L, (int)need);
+    }
+    if (!rc && L->profiling)
+        while (L->prof_ev.size() < L->prof_used + 2 * (size_t)nsteps) {
+            cudaEvent_t e;
+            FM_CUDA(cudaEventCreate(&e));
+            L->prof_ev.push_back(e);
+        }
+    return rc;
 }
 
 int probe_into(fm_lattice* L, double* dst)
@@ -1722,6 +1748,7 @@ int fm_step(fm_lattice* L, int nsteps)
     if (prc) return prc;
     if (L->mon_every > 0 && !one_launch_in_lanes(L))
         return fail(FM_ERR_UNSUPPORTED, "fm_step: the step monitor needs every boundary inside the fused step");
+    if ((prc = reserve_outputs(L, nsteps))) return prc;
     if (L->fuse_inlet && L->inlet_state == 0) prc = dispatch<InletFusedOp>(L);
     else if (!L->fuse_inlet && L->inlet_state == 1) prc = dispatch<InletPlainOp>(L);
     if (prc) return prc;
