@@ -2573,13 +2573,20 @@ int batch_launch_probes(fm_batch* B)
     return FM_OK;
 }
 
+bool batch_sampled(const fm_batch* B, long long s) { return B->probe_every > 0 && s % B->probe_every == 0; }
+
+// what may be read after step `s` of a run of steps, `last`: of its last (StepArgs::outputs)
+int batch_outputs(const fm_batch* B, long long s, bool last)
+{
+    return (last ? fm::kOutX0 : 0) | (last || batch_sampled(B, s) ? fm::kOutC : 0);
+}
+
 // one step of every lattice; `s` is the step number being completed
 int batch_one(fm_batch* B, long long s, int parity, bool last)
 {
-    const bool sampled = B->probe_every > 0 && s % B->probe_every == 0;
-    int rc = batch_dispatch_step(B, parity, (last ? fm::kOutX0 : 0) | (last || sampled ? fm::kOutC : 0));
+    int rc = batch_dispatch_step(B, parity, batch_outputs(B, s, last));
     if (rc) return rc;
-    if (sampled) return batch_launch_probes(B);
+    if (batch_sampled(B, s)) return batch_launch_probes(B);
     return FM_OK;
 }
 
@@ -2859,11 +2866,18 @@ int fm_batch_autotune(fm_batch* B, int trial_steps, int* mode, int* block, int* 
                 rc = fm_batch_set_mode(B, modes[im], blocks[ib], cpts[ic], pfs[ip]);
                 if (!rc) rc = batch_dispatch_const(B);
                 if (rc) break;
+                // the outputs of a run of steps (fm_batch_step), so mode 3, which leaves
+                // the others out, is timed as it runs
                 int parity = B->lats[0]->cur;
-                for (int i = 0; i < 2 && !rc; ++i, parity ^= 1) rc = batch_dispatch_step(B, parity, fm::kOutX0 | fm::kOutC);
+                long long s = B->lats[0]->step;
+                auto trial = [&](int n) {
+                    for (int i = 0; i < n && !rc; ++i, parity ^= 1, ++s)
+                        rc = batch_dispatch_step(B, parity, batch_outputs(B, s + 1, i + 1 == n));
+                };
+                trial(2);
                 if (rc) break;
                 cudaEventRecord(e0, B->stream);
-                for (int i = 0; i < trials && !rc; ++i, parity ^= 1) rc = batch_dispatch_step(B, parity, fm::kOutX0 | fm::kOutC);
+                trial(trials);
                 cudaEventRecord(e1, B->stream);
                 if (cudaEventSynchronize(e1) != cudaSuccess) { rc = fail(FM_ERR_CUDA, "autotune sync failed"); break; }
                 float ms = 0.0f;
