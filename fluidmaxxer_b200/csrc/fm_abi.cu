@@ -29,6 +29,7 @@
 #include <mutex>
 #include <string>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
 namespace fm_internal {
@@ -747,17 +748,47 @@ bool wide_offsets(const fm_lattice* L)
     return 18LL * L->ns + (long long)L->p.nx * L->p.ny + 2LL * L->p.nx + 1 >= (1LL << 31);
 }
 
+// Steps of even nx that keep the boundary planes in the boundary cells' own lanes.
+// What direct planes save is a launch's ramps (chaining) and the outputs nobody
+// reads; what they cost, stores of single elements, is per row and weighs more
+// once the populations are mostly in DRAM.  Time in lanes over time direct, sphere
+// packs, for runs of 20-40 steps
+//   FP32  nx 32: 3.0M cells 1.09, 4.0M 0.98, 5.0M 0.94, 18M 0.98; nx 48: 0.98-1.10
+//         up to 18M; nx 64: 1.03-1.19
+//   FP64  1.09 and more at every nx and size
+//   FP16  nx 32: 6.3M 1.01, 7.3M 0.93, 10.5M 0.90; nx 46: 6.3M 0.96; nx 160: 6.3M 1.02,
+//         7.3M 0.98, 10.5M 0.95; nx 256: 7.3M 1.02, 8.4M 0.99; nx 384: 9-22M 0.99-1.00;
+//         nx 448-512: 1.00-1.01; nx 640-1024: 1.01-1.03; 512x512x256 0.995
+//   FP16 + fixed point: as FP16 within 0.02
+//   BF16  nx 160: 5.2M 1.01, 6.3M 0.99, 10.5M 0.93; nx 256: 6.3M 1.01, 7.3M 0.98;
+//         nx 512: 7.3M 1.00, 8.4M 0.97, 33.5M 0.96; nx 1024: 9-22M 0.97-1.00
+// and for a step whose outputs may all be read, a call of one step above all
+//   FP32  nx 32: 2.5M 1.04, 3.5M 0.92, 5.0M 0.87; nx 64: 3.5M 1.01, 4.0M 0.98; nx 96:
+//         0.99-1.02 from 3M up; nx 128 and more: 1.02 and more
+//   FP64  1.10 and more
+//   FP16  nx 32: 1.0M 1.01, 2.5M 0.98, 6.0M 0.91; nx 96: 3.0M 1.00, 6.0M 0.93; nx 160:
+//         4.5M 1.00, 7.0M 0.95; nx 256: 6.0M 1.01, 8.0M 0.97; nx 512: 8.0M 1.00
+//   BF16  nx 32: 1.0M 0.96, 6.0M 0.91; nx 96: 2.0M 0.98, 6.0M 0.91; nx 160: 2.0M 1.02,
+//         3.5M 0.99, 6.0M 0.94; nx 256: 4.0M 1.00, 6.0M 0.98; nx 512: 5.0M 1.01, 6.0M 0.99
+template <typename T>
+bool planes_in_lanes(long long nx, long long n, int outputs)
+{
+    if (nx % 2 || sizeof(T) == 8) return false;
+    const bool all = outputs & fm::kOutX0;
+    if (sizeof(T) == 4) return all ? nx < 96 && n > 1800000 + 25000 * nx : nx < 48 && n > 3500000;
+    constexpr bool bf16 = std::is_same_v<T, __nv_bfloat16>;
+    if (all) return n > (bf16 ? std::min(15000 * nx, 4600000LL) : std::min(30000 * nx, 7000000LL));
+    if (n <= (nx < 192 ? 6000000 : 8000000) - (bf16 ? 1000000 : 0)) return false;
+    return bf16 || nx < 448 || n > 24000000;
+}
+
 // The fused planes written by their inward neighbours (fm::coupled_cell_direct):
 // when the pressure outlet and the AD Neumann outlet are both fused or both
 // absent, for rows that fit a warp's staging slots.
 template <typename T, typename QT>
 bool direct_planes(const fm::StepArgs<T, QT>& a)
 {
-    // 16-bit lattices of even nx beyond 24M cells keep the planes in their own
-    // lanes: FP16 512x256x256 sphere pack 1037 us a step against 1041-1046 with
-    // direct planes (512x256x128, 16.8M cells: 504 against 499)
-    if (sizeof(T) == 2 && a.nx % 2 == 0 && a.n > 24000000) return false;
-    return a.fuse_outlet == a.fuse_neumann && a.nx >= fm::kDirectMinNx;
+    return a.fuse_outlet == a.fuse_neumann && a.nx >= fm::kDirectMinNx && !planes_in_lanes<T>(a.nx, a.n, a.outputs);
 }
 
 // The direct-planes step runs blocks of 128 threads up to kSmallCells cells, where
