@@ -791,20 +791,22 @@ bool direct_planes(const fm::StepArgs<T, QT>& a)
     return a.fuse_outlet == a.fuse_neumann && a.nx >= fm::kDirectMinNx && !planes_in_lanes<T>(a.nx, a.n, a.outputs);
 }
 
-// The direct-planes step runs blocks of 128 threads up to kSmallCells cells, where
-// the last wave ends sooner: us a step with 128 and 256 threads, FP32 64x64x40 8.3
-// and 8.7, 128^3 76.0 and 76.8, 192x128x112 (2.8M) 97.9 and 96.6, 256x128x128 160
-// and 148; FP16 128^3 63.3 and 64.7, 436x124x206 390 and 339; FP64 128^3 137.7 and
-// 138.8, 436x124x206 704 and 699.  kResidentCells: what 148 SMs hold of the
-// 48-register forms at once.
+// The direct-planes step runs blocks of 128 threads up to kSmallCells cells and of
+// 256 above.  us a step with 128 and 256 threads: FP32 64x64x40 8.0 and 8.7, 128x96x80
+// 37.8 and 38.7, 128^3 (2.1M) 77.7 and 78.1, 160x128x112 (2.3M) 83.8 and 83.4,
+// 256x128x96 112.6 and 110.7, 256x128x128 168 and 151; FP16 128^3 64.7 and 66.3,
+// 256x128x96 90.6 and 92.7, 256x128x128 127.5 and 124.0, 256x192x160 289 and 256 (BF16
+// and FP16 + fixed point cross between the same two); FP64 128^3 138.9 and 140.3,
+// 256x192x160 499 and 501.  Small blocks end the last wave sooner; beyond some 200 MB of
+// populations read a step they lose more in DRAM.
 constexpr uint32_t kSmallCells = 2200000;
-constexpr uint32_t kResidentCells = 148 * 5 * 256;
 
 // `chained`: the previous work on `st` is a direct-planes step kernel of the
 // same run of steps, so this one may start while that one drains (programmatic
 // dependent launch; the kernel waits for it before its first pull).  Measured
-// 2-4 us a step, what a launch and the first and last blocks' ramps cost: FP32
-// 32x16x16 6.2 -> 4.2 us, 128x64x64 24.6 -> 22.3, 256x128x128 164 -> 161.
+// 1-2 us a step, what a launch and the first and last blocks' ramps cost: FP32
+// 32x16x16 6.2 -> 3.8 us, 64x32x32 6.3 -> 4.9, 128x64x64 22.6 -> 21.3, 256x128x128
+// 158 -> 156.
 template <typename T, typename QT, bool POROUS, bool MON>
 void launch_coupled(const fm_lattice* L, int grid, cudaStream_t st, const fm::StepArgs<T, QT>& a, bool chained = false)
 {
@@ -818,7 +820,7 @@ void launch_coupled(const fm_lattice* L, int grid, cudaStream_t st, const fm::St
             const int block = cells <= kSmallCells ? kBlock / 2 : kBlock;
             fm::StepArgs<T, QT> ad = a;
             ad.pf_dist *= (uint32_t)(kBlock / block);
-            ad.early = L->elt >= 4 && cells > kResidentCells;
+            ad.early = L->elt >= 4 && cells > kSmallCells;
             cudaLaunchAttribute attr{};
             attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
             attr.val.programmaticStreamSerializationAllowed = 1;

@@ -370,7 +370,7 @@ struct StepArgs {
     int* __restrict__ status;             // device status word: bit 0 a shared-memory stage wait gave up
     // direct planes only:
     int outputs;                          // what may be read before the next step: kOutX0 x0post, kOutC the C of every cell
-    int early;                            // the grid is more than one resident wave
+    int early;                            // the next step's blocks may be placed before this grid's end
     uint32_t rest;                        // kRest: both buffers hold resting obstacles' populations; 0: all are written
 };
 
@@ -1480,10 +1480,12 @@ __device__ __forceinline__ void coupled_cell_direct(const StepArgs<T, QT>& a, ui
         }
     }
     // The next step's blocks may take their places; they wait for this grid's end
-    // before their pulls.  Not in a grid that is resident as a whole (its blocks'
-    // ends let the next grid in): blocks placed beside running ones pile up on few
-    // SMs (64x32x32: 8.2 us a step with the trigger at the start, 5.4 here, 4.9
-    // with none; 128x64x64: 20.7 here, 21.0 with none).
+    // before their pulls.  Only in large FP32 and FP64 grids: in small ones blocks
+    // placed beside running ones pile up on few SMs, and their own blocks' ends let
+    // the next grid in.  us a step without and with: FP32 64x64x32 6.5 and 7.6,
+    // 96x64x48 11.6 and 12.0, 128x64x64 20.8 and 21.2, 128^3 78.6 and 78.4, 256x256x128
+    // 298.8 and 297.7, 512x256x256 1155 and 1152; FP64 64x64x44 12.0 and 12.4,
+    // 128x64x64 37.2 and 37.5, 256x256x128 532.7 and 530.2, 512x256x256 2154 and 2144.
     if (a.early) pdl_launch_dependents();
     bool st_own = active && moving;      // the lane stores its own cell's f
     uint32_t near0 = 0u, nearn = 0u;     // lanes at x = 1 (inlet) and x = nx-2 (outlet)

@@ -1,8 +1,8 @@
 """Odd row lengths at the sizes where the direct-planes step changes its launch:
-beyond 189,440 cells the next step's blocks are placed while this one still
-stores, beyond 2.2M cells blocks hold 256 threads, at both the flag words are
-fetched ahead; and a 16-bit lattice whose pulls need unsigned offsets.  Boundary
-cells and their neighbours fall into different warps and blocks throughout."""
+several resident waves, with the flag words fetched ahead; beyond 2.2M cells,
+blocks of 256 threads and the next step's blocks placed while this one still
+stores; and a 16-bit lattice whose pulls need unsigned offsets.  Boundary cells
+and their neighbours fall into different warps and blocks throughout."""
 import dataclasses
 
 import numpy as np
