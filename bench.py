@@ -31,7 +31,7 @@ import numpy as np
 ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
-BYTES_PER_CELL = {"f32": 216, "f16": 120, "bf16": 120, "f16q": 120, "f64": 432}   # algorithmic bytes per coupled cell update
+BYTES_PER_CELL = {"f32": 216, "f16": 120, "bf16": 120, "f16q": 120, "f64": 432}   # algorithmic bytes per coupled cell update (step_bytes)
 BYTES_PER_POP = {"f32": 4, "f16": 2, "bf16": 2, "f16q": 2, "f64": 8}
 FALLBACK_HBM_GBS = 6650.0
 
@@ -48,7 +48,7 @@ def parse():
     ap.add_argument("--size", default=None, help="override lattice size, e.g. 256x128x128")
     ap.add_argument("--prefetch", type=int, default=None,
                     help="L2 prefetch distance of the step kernel in 256-cell blocks (0 off; default: the "
-                         "library's choice, half a resident wave for f32 and none for the other forms)")
+                         "library's choice)")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-e2e", action="store_true")
     ap.add_argument("--shard", action="store_true",
@@ -106,6 +106,26 @@ def traffic_per_cell(precision):
         if m:
             return float(m.group(1))
     return None
+
+
+def resting_cells(p, precision):
+    """Cells whose D3Q19 populations the step does not move: whole 32-byte sectors
+    of obstacles, two cells or more from an x-face, which stay at rest from the
+    start (FP32 and FP64 steps of BGK lattices with rows of 16 cells up)."""
+    if precision not in ("f32", "f64") or p.collision != "bgk" or p.nx < 16:
+        return 0
+    g = 32 // BYTES_PER_POP[precision]
+    solid = np.asarray(p.solid).reshape(-1)
+    groups = solid[: solid.size // g * g].reshape(-1, g).all(axis=1)
+    lo = (np.arange(groups.size, dtype=np.int64) * g) % p.nx
+    return int(g * np.count_nonzero(groups & (lo >= 2) & (lo + g - 1 <= p.nx - 3)))
+
+
+def step_bytes(p, precision, rest=True):
+    """Algorithmic bytes of one step: every cell's, less both transfers of the
+    resting cells' D3Q19 populations (`rest`: the step leaves them out)."""
+    resting = resting_cells(p, precision) if rest else 0
+    return BYTES_PER_CELL[precision] * p.n_cells - 2 * 19 * BYTES_PER_POP[precision] * resting
 
 
 class Clocks:
@@ -341,9 +361,10 @@ def run_sharded(args, p, world, rank, local, stream, barrier, max_over_ranks):
     L.close()
     n = p.n_cells
     peak, peak_kind = measured_peak()
-    bpc = BYTES_PER_CELL[args.precision]
+    per_step = step_bytes(p, args.precision)
+    bpc = per_step / n
     # per GPU: its own cells' algorithmic bytes over the whole step time
-    achieved = bpc * (n / world) * args.steps / (el_ms / 1e3) / 1e9
+    achieved = per_step / world * args.steps / (el_ms / 1e3) / 1e9
     halo = sr.io.nbytes
     return {
         "metric": "coupled NS+AD MLUPS", "value": n * args.steps / (el_ms / 1e3) / 1e6, "unit": "MLUPS",
@@ -476,8 +497,9 @@ def run_batch(args, world, rank, stream, barrier, max_over_ranks):
         L.close()
     value = total_cells * args.steps / (el_ms / 1e3) / 1e6
     peak, peak_kind = measured_peak()
-    bpc = BYTES_PER_CELL[args.precision]
-    achieved = bpc * cells * args.steps / (el_ms / 1e3) / 1e9
+    per_step = sum(step_bytes(p, args.precision, rest=cfg["mode"] == 3) for p in ps)
+    bpc = per_step / cells
+    achieved = per_step * args.steps / (el_ms / 1e3) / 1e9
     sizes = sorted({(p.nx, p.ny, p.nz) for p in all_ps})
     return {
         "metric": "coupled NS+AD MLUPS", "value": value, "unit": "MLUPS", "n_gpus": world,
@@ -534,8 +556,9 @@ def time_form(p, prec, args, stream, max_over_ranks, f32_value, peak, peak_kind,
     Lp.close()
     mlups = n * args.steps * world / (ms / 1e3) / 1e6
     per_launch = kern_ms / max(launches, 1)
-    bpc = BYTES_PER_CELL[prec]
-    achieved = bpc * n / (per_launch / 1e3) / 1e9 if per_launch > 0 else 0.0
+    per_step = step_bytes(p, prec)
+    bpc = per_step / n
+    achieved = per_step / (per_launch / 1e3) / 1e9 if per_launch > 0 else 0.0
     pc_gbs = pc_bytes / (pc_ms / 1e3) / 1e9
     out = {"value": mlups, "unit": "MLUPS", "speedup_vs_f32": mlups / f32_value, "layout": layout,
            "kernel": kernel,
@@ -584,7 +607,7 @@ def time_pair_kernels(p, prec, args, stream, max_over_ranks, peak):
 def time_batch_form(args, stream, max_over_ranks, f32_value, peak, peak_kind, world, samples=64):
     """The batching form on its own workload (64 uneven porous samples, edges
     from {96..160}^3, per-sample Langmuir parameters, FP32), autotuned, timed
-    over the bench's step count after its warm-up; roofline at 216 B per cell."""
+    over the bench's step count after its warm-up; roofline at step_bytes."""
     import torch
 
     from fluidmaxxer_b200 import lattice, problems
@@ -606,11 +629,12 @@ def time_batch_form(args, stream, max_over_ranks, f32_value, peak, peak_kind, wo
     for L in lats:
         L.close()
     mlups = cells * args.steps * world / (ms / 1e3) / 1e6
-    achieved = BYTES_PER_CELL["f32"] * cells * args.steps / (ms / 1e3) / 1e9
+    per_step = sum(step_bytes(q, "f32", rest=cfg["mode"] == 3) for q in ps)
+    achieved = per_step * args.steps / (ms / 1e3) / 1e9
     return {"value": mlups, "unit": "MLUPS", "workload": f"batch of {samples} samples, {cells} cells",
             "autotuned": cfg, "ms_per_step": ms / args.steps,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                         "peak_source": peak_kind, "algorithmic_bytes_per_cell": BYTES_PER_CELL["f32"],
+                         "peak_source": peak_kind, "algorithmic_bytes_per_cell": per_step / cells,
                          "kernel": "the whole batch step (all launches and probes)"}}
 
 
@@ -727,8 +751,9 @@ def main():
     n = p.n_cells
     value = job_mlups(n, args.steps, world, el_ms)
     peak, peak_kind = measured_peak()
-    bpc = BYTES_PER_CELL[args.precision]
-    achieved = bpc * n * launches / (kern_ms / 1e3) / 1e9 if kern_ms > 0 else 0.0
+    per_step = step_bytes(p, args.precision, rest=main_kernel == "k_coupled_step")
+    bpc = per_step / n
+    achieved = per_step * launches / (kern_ms / 1e3) / 1e9 if kern_ms > 0 else 0.0
     tpc = traffic_per_cell(args.precision) if main_kernel == "k_coupled_step" else None
     line = {
         "metric": "coupled NS+AD MLUPS", "value": value, "unit": "MLUPS", "n_gpus": world,
