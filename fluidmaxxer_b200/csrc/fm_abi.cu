@@ -160,7 +160,7 @@ struct fm_lattice {
     int fuse_outlet = 0, fuse_neumann = 0, fuse_dirichlet = 0;
     uint32_t pf_dist = 0;               // L2 prefetch distance of the fused kernel (blocks)
     uint32_t pf_full = 0;               // the same for the in-lane planes' kernels
-    bool pf_set = false;                // pf_dist fixed by fm_set_tuning
+    bool pf_set = false;                // pf_dist fixed by fm_set_prefetch_distance
     double rho_out = 1.0, c_in = 0.0;
     bool profiling = false;
     double* d_wide = nullptr;           // FP64 staging plane of the field getters

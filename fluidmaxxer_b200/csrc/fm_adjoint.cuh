@@ -187,8 +187,8 @@ constexpr int kAdjThreads = 128;
 template <typename T>
 constexpr int kAdjBlocks = sizeof(T) == 8 ? 3 : 6;
 
-// Bound by latency and instruction issue (24 FP32 warps an SM, 2600 instructions
-// each).  It replaces a cell kernel, a stream kernel and an inlet kernel, which
+// Bound by latency and instruction issue (24 FP32 warps an SM, 2520 instructions
+// each, 48% of cycles issuing).  It replaces a cell kernel, a stream kernel and an inlet kernel, which
 // passed the 26 adjoint planes through memory once more (564 against 352 B a
 // cell), formed every product with the zero velocity components and took the
 // neighbour table in every warp.  All loads of populations and adjoints come
