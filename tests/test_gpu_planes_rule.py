@@ -34,3 +34,24 @@ def test_same_state_as_monitored_steps(prec, size):
             assert np.array_equal(got[k], ref[k]), k
     a.close()
     b.close()
+
+
+def test_batch_equals_single_lattices():
+    """Mode 3 of a batch takes the same rule: here only the steps whose outputs may
+    be read, the last of a call or of a replayed graph, take the lanes."""
+    sizes = [(64, 176, 178), (96, 176, 178)]
+    solo = [lattice.from_problem(problems.channel_small(5, *s), "f16") for s in sizes]
+    both = [lattice.from_problem(problems.channel_small(5, *s), "f16") for s in sizes]
+    B = lattice.Batch(both)
+    B.set_config(mode=3)
+    for steps in (1, 5, 4):
+        B.step(steps)
+        B.synchronize()
+        for a, b in zip(solo, both):
+            a.step(steps)
+            got, ref = b.fields(dtype=np.float32), a.fields(dtype=np.float32)
+            for k in ref:
+                assert np.array_equal(got[k], ref[k]), (k, steps)
+    B.close()
+    for L in solo + both:
+        L.close()
